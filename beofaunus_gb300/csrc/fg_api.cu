@@ -139,6 +139,8 @@ struct fg_system {
     int cnt_accepted_host = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     size_t device_bytes = 0;
+    void *work64 = nullptr;        // FP64 energies and g(r): grown when needed (ensure_work64)
+    size_t work64_cap = 0;
 };
 
 namespace {
@@ -148,7 +150,7 @@ void free_all(fg_system *h) {
                     h->p_cell, h->p_slot, h->cell_pos, h->kvec, h->core_tab, h->core_tab2, h->kpack, h->qfix,
                     h->qnew, h->sc, h->trial_out, h->corr, h->pair_part, h->req, h->dp_fix, h->sc_tab, h->trials,
                     h->log_du, h->log_acc, h->kseg, h->rb_items, h->raw_idx, h->raw_disp, h->raw_u,
-                    h->eb_ranges, h->cl_items, h->d_desc_cl};
+                    h->eb_ranges, h->cl_items, h->d_desc_cl, h->work64};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -1699,8 +1701,8 @@ int64_t fg_device_bytes(fg_system *h) { return h ? (int64_t)h->device_bytes : 0;
 #include "fg_noalloc.cu"
 #include "fg_mol.cu"
 #include "fg_tune.cu"
+#include "fg_energy64.cu"
 #include "fg_rdf.cu"
 #include "fg_state.cu"
-#include "fg_energy64.cu"
 #include "fg_volume.cu"
 #include "fg_dip.cu"
