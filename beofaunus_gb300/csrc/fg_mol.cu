@@ -9,31 +9,51 @@
 // Included by fg_api.cu (one translation unit).
 //
 // Work split. One system runs on a thread-block cluster of C CTAs (C <= 16,
-// one per SM). A trial moves one molecule of gs sites; its energy change is a
-// sum over the gs moved sites against all N - gs other sites. CTA r owns the
-// site slice [r N/C, (r+1) N/C) and the dipole-site slice [r D/C, (r+1) D/C),
-// kept in its shared memory, and sums its part; the C partial sums meet
-// through distributed shared memory after one cluster barrier per trial, and
-// every CTA then makes the same Metropolis decision from the same numbers.
-// Each CTA keeps its own replica of the FP64-exact state (64-bit fixed-point
+// one per SM). CTA r owns the site slice [r N/C, (r+1) N/C) and the
+// dipole-site slice [r D/C, (r+1) D/C), kept in its shared memory. Trials run in groups of up to
+// kMolAhead, as the ion kernels run blocks (fg_dh_block.cu): every trial of the
+// group is evaluated against the configuration at the group's start, one warp
+// per trial and CTA, so that nothing but the warp's own sums happens per
+// trial; if trial a was accepted, a later trial m of the group (another
+// molecule) differs from that value by
+//     c(a, m) = [u(n_m, n_a) - u(o_m, n_a)] - [u(n_m, o_a) - u(o_m, o_a)]
+// over the two molecules' site pairs, which the cluster's warps evaluate for
+// all a < m. The C partial sums and the c(a, m) meet in every CTA's shared
+// memory (remote stores, one cluster barrier per group), every CTA resolves
+// the group in order with the same numbers, and a trial whose molecule an
+// accepted trial of the group moved ends the group (it is evaluated again in
+// the next one): decisions are those of the one-trial-at-a-time chain. Each
+// CTA keeps its own replica of the FP64-exact state (64-bit fixed-point
 // positions, FP64 dipole vectors, mass centres) in global memory, so no CTA
 // ever reads what another CTA wrote during the sweep.
+//
+// What bounds it: instruction issue in the pair loops (of 25 us per trial at
+// 1000 x 20 sites on 4 CTAs the loop over far sites takes 9.5, image edges 1.8,
+// near pairs 2.7, corrections 2, set-up 0.8). One trial at a time, six integer
+// differences converted per pair and seven block barriers per trial took 50 us
+// on 4 CTAs and 19 us on 16 (now 9).
 //
 // Precision. Positions are 64-bit fixed point (X = x/L 2^64). The rotation
 // of a trial runs in FP64 on offsets from the rotation centre (20 sites per
 // trial). Pair terms are FP32 except where that would exceed the 1e-6 kT
 // budget:
-//  * far pairs (both r_old, r_new >= rc): LJ and ion-dipole are small; LJ
-//    uses 22-bit-truncated coordinate differences converted without the
-//    conversion pipe, ion-dipole exact 32-bit differences;
-//  * near pairs (r_old or r_new < rc) are queued and evaluated afterwards,
-//    densely: LJ and Coulomb as differences u(r_new) - u(r_old) whose
+//  * far pairs (both r_old, r_new >= rc): LJ and ion-dipole are small. Site j
+//    is taken relative to the moved molecule's old mass centre (the 32-bit
+//    minimum-image difference D_j, converted once per trial), site i as its
+//    offset delta_i from that centre, so that a pair costs no conversion: D_j's
+//    rounding is common to the old and the new position and its effect on
+//    u_new - u_old cancels to first order;
+//  * near pairs (r_old or r_new < rc) are queued and evaluated 32 at a time:
+//    LJ and Coulomb as differences u(r_new) - u(r_old) whose
 //    rounding error scales with the difference, from r_new^2 - r_old^2
-//    computed in FP64 from exact 48-bit coordinate differences; terms with a
-//    dipole in FP64 (a few per trial);
+//    computed from exact coordinate differences; terms with a dipole in FP32
+//    (a few per trial);
 //  * per-trial sums are double-float (df).
-// The image convention is the reference's minimum image (Cuboid::vdist),
-// taken on exact integer differences.
+// The image convention is the reference's minimum image (Cuboid::vdist). For a
+// site with |D| + max |delta| < L/2 on each axis D - delta is the minimum
+// image of every pair; the others (19 % at 1000 molecules in 150 A) are
+// collected and take min(|dx|, L - |dx|) for LJ and the exact integer
+// difference for ion-dipole, which is odd in r.
 namespace fgm {
 
 using fg::df;
@@ -45,8 +65,14 @@ using fg::warp_sum_df;
 
 constexpr int kMolThreads = 512;
 constexpr int kMaxGroupSites = 31;   // lane gs of the setup warp computes the mass centre
-constexpr int kQueueCap = 3072;
 constexpr int kMaxCluster = 16;
+constexpr int kMolAhead = 16;   // trials of a group, one per warp
+constexpr int kMolWarps = kMolThreads / 32;
+constexpr int kMolPerLane = 4;  // sites per lane of the far loop
+constexpr int kMolSiteQueue = 32 * (kMolPerLane + 1);   // a queue of less than 32 sites takes one more turn
+constexpr int kMolPairQueue = 256;   // near pairs of a warp (about 110 at C = 16 and 425 at C = 4 for 1000 x 20
+                                     // sites; what exceeds it the warp evaluates as it comes)
+constexpr int kMolQueue = 2 * kMolSiteQueue + kMolPairQueue;   // words of a warp: two site queues, near pairs
 
 // Error bits
 constexpr int kMolErrNonFinite = 8;
@@ -120,13 +146,11 @@ __device__ __forceinline__ unsigned cluster_size() {
 __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Load a float2 from the shared memory of CTA `rank` of this cluster.
-__device__ __forceinline__ float2 ld_cluster_f2(const float2 *p, unsigned rank) {
+// Store a float2 into the shared memory of CTA `rank` of this cluster.
+__device__ __forceinline__ void st_cluster_f2(float2 *p, unsigned rank, float2 v) {
     unsigned a = (unsigned)__cvta_generic_to_shared(p), ra;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
-    float2 v;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(ra) : "memory");
-    return v;
+    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(ra), "f"(v.x), "f"(v.y) : "memory");
 }
 
 // ---------------------------------------------------------------- helpers
@@ -152,70 +176,89 @@ __device__ __forceinline__ D3 qrot(double w, const D3 &v, const D3 &p) {
 }
 
 // ---------------------------------------------------------------- shared memory
-// Moved-molecule data, double-buffered: while the CTA sums trial t, the last
-// warp prepares trial t+1 (its rotation runs in FP64 and is latency-bound).
+// Moved-molecule data of one trial of the group, set up by one warp (the
+// rotations run in FP64, 1/64 of the FP32 rate: sixteen side by side take a
+// quarter of what they take one after the other).
 struct GroupBuf {
     int4 *go, *gn;    // old/new high words; .w = type | dipole flag (go) / site << 8 | type (gn)
-    float4 *gfo;      // old dipole vector mu-hat * mu (x, y, z), mu
+    float4 *gfo;      // old dipole vector mu-hat * mu (x, y, z), mu (sites with a dipole)
     float4 *gfn;      // new dipole vector
+    float4 *dlo;      // old offset from the reference point (Angstrom), .w = its square
+    float4 *dln;      // new offset
     double *gmu;      // [gs][3] new unit dipole (FP64, for the replica)
     int64_t *gX;      // [gs][3] new fixed-point positions
     int64_t *gcm;     // [3] new mass centre
+    float4 *lim;      // half box less the largest |offset| per axis; .w = squared distance from the
+                      // reference point beyond which no pair of the molecule is near
+    int4 *ref;        // reference point (high words of the old mass centre), .w = sites with a dipole
+    uint32_t *qmask;  // sites with a charge
 };
 
 struct MolSmem {
     int4 *spos;     // site slice: high words, .w = type
     float4 *sdip;   // dipole slice: mu-hat * mu, mu
     int4 *sdpos;    // dipole slice positions, .w = site << 8 | type
-    GroupBuf buf[2];
-    uint32_t *queue;
-    int *qcount;
-    float2 *red;   // [32]
-    float2 *part;  // [2] cluster partial sums (double-buffered by trial parity)
-    int *flag;     // [4]: decision, speculation invalid
+    unsigned char *groups;   // `ahead` group buffers
+    uint32_t *queue;   // [kMolWarps][kMolQueue]: a warp's sites that may change image, near sites, near pairs
+    float2 *part;      // [2][kMaxCluster][kMolWarps] partial sums of the cluster's warps (by group parity)
+    float2 *corr;      // [2][kMolAhead][kMolAhead] c(a, m)
+    float *lbq;        // [16] lB q of each type
+    int *info;         // [4] resolved, accepted, stop
+    int *npair;        // [kMolWarps] near pairs queued by each warp
 };
 
 __host__ __device__ inline size_t mol_align16(size_t x) { return (x + 15) & ~(size_t)15; }
 
 __host__ __device__ inline size_t mol_group_bytes(int gs) {
-    return mol_align16((size_t)gs * 16 * 4) + mol_align16((size_t)gs * 3 * 8 * 2 + 3 * 8);
+    return mol_align16((size_t)gs * 16 * 6) + mol_align16((size_t)gs * 3 * 8 * 2 + 3 * 8) + 48;
 }
 
-__host__ __device__ inline void mol_smem_layout(int ns, int nd, int gs, bool slice_smem, size_t off[16]) {
+__host__ __device__ inline void mol_smem_layout(int ns, int nd, int gs, bool slice_smem, int ahead, size_t off[16]) {
     size_t o = 0;
     off[0] = o; o += mol_align16(slice_smem ? (size_t)ns * 16 : 0);   // spos
     off[1] = o; o += mol_align16((size_t)nd * 16);                    // sdip
     off[2] = o; o += mol_align16((size_t)nd * 16);                    // sdpos
-    off[3] = o; o += 2 * mol_group_bytes(gs);                         // group buffers
-    off[4] = o; o += mol_align16((size_t)kQueueCap * 4 + 16);         // queue, qcount
-    off[5] = o; o += mol_align16(32 * 8 + 2 * 8 + 16);                // red, part, flag
-    off[6] = o;
+    off[3] = o; o += ahead * mol_group_bytes(gs);                     // group buffers
+    off[4] = o; o += (size_t)kMolWarps * kMolQueue * 4;               // queue
+    off[5] = o; o += (size_t)2 * kMaxCluster * kMolWarps * 8;         // part
+    off[6] = o; o += (size_t)2 * kMolAhead * kMolAhead * 8 + 64 + 16 + 4 * kMolWarps;   // corr, lbq, info, npair
+    off[7] = o;
 }
 
-__device__ inline MolSmem mol_carve(unsigned char *base, int ns, int nd, int gs, bool slice_smem) {
+__device__ inline MolSmem mol_carve(unsigned char *base, int ns, int nd, int gs, bool slice_smem, int ahead) {
     size_t off[16];
-    mol_smem_layout(ns, nd, gs, slice_smem, off);
+    mol_smem_layout(ns, nd, gs, slice_smem, ahead, off);
     MolSmem s;
     s.spos = (int4 *)(base + off[0]);
     s.sdip = (float4 *)(base + off[1]);
     s.sdpos = (int4 *)(base + off[2]);
-    for (int b = 0; b < 2; b++) {
-        unsigned char *g = base + off[3] + b * mol_group_bytes(gs);
-        GroupBuf &B = s.buf[b];
-        B.go = (int4 *)g;
-        B.gn = B.go + gs;
-        B.gfo = (float4 *)(B.gn + gs);
-        B.gfn = B.gfo + gs;
-        B.gmu = (double *)(g + mol_align16((size_t)gs * 16 * 4));
-        B.gX = (int64_t *)(B.gmu + 3 * gs);
-        B.gcm = B.gX + 3 * gs;
-    }
+    s.groups = base + off[3];
     s.queue = (uint32_t *)(base + off[4]);
-    s.qcount = (int *)(s.queue + kQueueCap);
-    s.red = (float2 *)(base + off[5]);
-    s.part = s.red + 32;
-    s.flag = (int *)(s.part + 2);
+    s.part = (float2 *)(base + off[5]);
+    s.corr = (float2 *)(base + off[6]);
+    s.lbq = (float *)(s.corr + 2 * kMolAhead * kMolAhead);
+    s.info = (int *)(s.lbq + 16);
+    s.npair = s.info + 4;
     return s;
+}
+__device__ __forceinline__ GroupBuf mol_group(const MolSmem &s, int gs, int b) {
+    unsigned char *g = s.groups + b * mol_group_bytes(gs);
+    GroupBuf B;
+    B.go = (int4 *)g;
+    B.gn = B.go + gs;
+    B.gfo = (float4 *)(B.gn + gs);
+    B.gfn = B.gfo + gs;
+    B.dlo = B.gfn + gs;
+    B.dln = B.dlo + gs;
+    g += mol_align16((size_t)gs * 16 * 6);
+    B.gmu = (double *)g;
+    B.gX = (int64_t *)(B.gmu + 3 * gs);
+    B.gcm = B.gX + 3 * gs;
+    g += mol_align16((size_t)gs * 3 * 8 * 2 + 3 * 8);
+    B.lim = (float4 *)g;
+    B.ref = (int4 *)(g + 16);
+    B.qmask = (uint32_t *)(g + 32);
+    return B;
 }
 
 // ---------------------------------------------------------------- pair terms
@@ -223,22 +266,6 @@ __device__ __forceinline__ float rcp_approx(float x) {
     float y;
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
-}
-
-// Far pairs: squared distance from the high-word differences rounded to
-// float (relative error < 1e-7; one conversion per axis, which measured
-// faster than a shift-and-add conversion on the integer pipe).
-__device__ __forceinline__ float far_r2(int4 a, int4 b, float3 sc9) {
-    // the 32-bit minimum-image difference rounded to float (sc9 / 512 = L / 2^32)
-    const float dx = (float)wsub(a.x, b.x) * (sc9.x * (1.0f / 512.0f));
-    const float dy = (float)wsub(a.y, b.y) * (sc9.y * (1.0f / 512.0f));
-    const float dz = (float)wsub(a.z, b.z) * (sc9.z * (1.0f / 512.0f));
-    return fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-}
-__device__ __forceinline__ float lj_r2(float r2, float s2, float e4) {
-    const float x = s2 * rcp_approx(r2);
-    const float x3 = x * x * x;
-    return e4 * fmaf(x3, x3, -x3);
 }
 
 // Exact 32-bit difference vector a - b in Angstrom (FP32).
@@ -336,6 +363,9 @@ __device__ __noinline__ float near_pair_b(int4 po, int4 pn, float4 fo, float4 fn
     float acc = d.lB * qi * (dot3f(v, rn) * in_ * in_ * in_ - dot3f(v, ro) * io * io * io);
     if (po.w & 0x100) {
         auto dd = [&](float4 f, float3 r, float r2, float ri, int4 p) {
+            // far pairs (a group's corrections pass them) first: the integer
+            // squares of three half boxes would not fit 63 bits
+            if (!(r2 < d.rc2near)) return 0.0f;
             const int dx = wsub(p.x, pk.x), dy = wsub(p.y, pk.y), dz = wsub(p.z, pk.z);
             bool inside;
             if (d.cubic) {
@@ -361,18 +391,22 @@ __device__ __noinline__ float near_pair_b(int4 po, int4 pn, float4 fo, float4 fn
 
 // ---------------------------------------------------------------- trial setup
 // New coordinates of the moved molecule: FP64 rotation of offsets from the
-// centre, then translation, one lane per site; lane gs does the mass centre.
-// Old data come from this CTA's replica. Called by one warp.
-__device__ __forceinline__ void setup_trial(const MolTrial &tr, const MolDesc &d, const GroupBuf &B, int rank,
-                                            int lane) {
+// centre, then translation. Items are spread over the warp's lanes: the gs
+// sites, the mass centre, and the dipoles of the sites that carry one, so
+// that positions and dipoles rotate in the same FP64 instructions. Old data
+// come from this CTA's replica. Called by one warp.
+__device__ __noinline__ void setup_trial(const MolTrial &tr, const MolDesc &d, const GroupBuf &B, int rank) {
+    const int lane = threadIdx.x & 31;
     const int gs = d.gs, g = tr.g;
     const int64_t *P = d.rep_pos + (size_t)rank * d.N * 3;
     const double *MU = d.rep_mu + (size_t)rank * d.N * 3;
     const int64_t *CM = d.rep_cm + (size_t)rank * d.M * 3;
-    if (lane > gs) return;
-    const bool explicit_ = tr.flags & 4;
+    const bool explicit_ = tr.flags & 4, rot = (tr.flags & 1) && !explicit_, trans = (tr.flags & 2) && !explicit_;
+    const float3 s32 = make_float3(d.s32[0], d.s32[1], d.s32[2]);
     int64_t c[3] = {0, 0, 0};
-    if (!explicit_) {
+    int rf[3];
+    for (int a = 0; a < 3; a++) rf[a] = hi32(CM[3 * g + a]);
+    if (rot) {
         if (tr.center == 0) {
             for (int a = 0; a < 3; a++) c[a] = CM[3 * g + a];
         } else {
@@ -380,295 +414,661 @@ __device__ __forceinline__ void setup_trial(const MolTrial &tr, const MolDesc &d
             for (int a = 0; a < 3; a++) c[a] = P[3 * cs + a];
         }
     }
+    // this lane's site: type, dipole, charge
+    const int my = g * gs + min(lane, gs - 1);
+    int type = 0;
+    bool has_mu = false, has_dip = false, has_q = false;
+    if (lane < gs) {
+        type = d.pos4[my].w & 0xFF;
+        has_dip = d.site_dip[my] >= 0;
+        has_q = d.qtype[type] != 0.0f;
+        unsigned long long bits = 0;   // a nonzero dipole unit vector (compared as integers, off the FP64 pipe)
+        for (int a = 0; a < 3; a++) bits |= (unsigned long long)__double_as_longlong(MU[3 * my + a]) << 1;
+        if (explicit_ && d.expl_mu) bits = 1;
+        has_mu = bits != 0;
+        if (!has_mu) {
+            for (int a = 0; a < 3; a++) B.gmu[3 * lane + a] = MU[3 * my + a];
+            if (has_dip) B.gfo[lane] = B.gfn[lane] = make_float4(0.0f, 0.0f, 0.0f, (float)d.mus[my]);
+        }
+    }
+    const uint32_t hm = __ballot_sync(0xffffffffu, has_mu), hd = __ballot_sync(0xffffffffu, has_dip);
+    const uint32_t hq = __ballot_sync(0xffffffffu, has_q);
     const D3 qv = {tr.qx, tr.qy, tr.qz};
-    auto move_point = [&](const int64_t X[3], int64_t out[3]) {
-        int64_t Y[3] = {X[0], X[1], X[2]};
-        if (tr.flags & 1) {
-            const D3 a = {(double)(int64_t)((uint64_t)X[0] - (uint64_t)c[0]) * d.s64d[0],
-                          (double)(int64_t)((uint64_t)X[1] - (uint64_t)c[1]) * d.s64d[1],
-                          (double)(int64_t)((uint64_t)X[2] - (uint64_t)c[2]) * d.s64d[2]};
-            const D3 b = qrot(tr.qw, qv, a);
-            Y[0] = (int64_t)((uint64_t)c[0] + (uint64_t)__double2ll_rn(b.x * d.inv64d[0]));
-            Y[1] = (int64_t)((uint64_t)c[1] + (uint64_t)__double2ll_rn(b.y * d.inv64d[1]));
-            Y[2] = (int64_t)((uint64_t)c[2] + (uint64_t)__double2ll_rn(b.z * d.inv64d[2]));
+    const int nit = gs + 1 + __popc(hm);
+    float4 dlo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), dln = dlo;   // the lane's site offsets (item = lane < gs)
+    for (int b0 = 0; b0 < nit; b0 += 32) {
+        const int it = b0 + lane;
+        const bool dip = it > gs && it < nit, pos = it <= gs;
+        int src = it;
+        if (dip) {   // the (it - gs - 1)-th site with a dipole vector
+            uint32_t m = hm;
+            for (int k = it - gs - 1; k > 0; k--) m &= m - 1;
+            src = __ffs(m) - 1;
         }
-        if (tr.flags & 2)
-            for (int a = 0; a < 3; a++) Y[a] = (int64_t)((uint64_t)Y[a] + (uint64_t)tr.t[a]);
-        for (int a = 0; a < 3; a++) out[a] = Y[a];
-    };
-    if (lane == gs) {
-        int64_t cn[3];
-        if (explicit_) {
-            for (int a = 0; a < 3; a++) cn[a] = d.expl_cm ? d.expl_cm[a] : CM[3 * g + a];
-        } else {
-            const int64_t co[3] = {CM[3 * g], CM[3 * g + 1], CM[3 * g + 2]};
-            move_point(co, cn);
+        const int site = g * gs + src;
+        D3 v = {0.0, 0.0, 0.0};
+        int64_t X[3] = {0, 0, 0};
+        if (dip) {
+            v = {MU[3 * site], MU[3 * site + 1], MU[3 * site + 2]};
+        } else if (pos) {
+            const int64_t *S = it < gs ? P + 3 * site : CM + 3 * g;
+            for (int a = 0; a < 3; a++) X[a] = S[a];
+            if (rot)
+                v = {(double)(int64_t)((uint64_t)X[0] - (uint64_t)c[0]) * d.s64d[0],
+                     (double)(int64_t)((uint64_t)X[1] - (uint64_t)c[1]) * d.s64d[1],
+                     (double)(int64_t)((uint64_t)X[2] - (uint64_t)c[2]) * d.s64d[2]};
         }
-        for (int a = 0; a < 3; a++) B.gcm[a] = cn[a];
-        return;
+        D3 w = v;
+        if (rot) w = qrot(tr.qw, qv, v);   // positions, and DipoleParticle::rotate (point.h:672-679)
+        if (dip) {
+            if (explicit_ && d.expl_mu) w = {d.expl_mu[3 * src], d.expl_mu[3 * src + 1], d.expl_mu[3 * src + 2]};
+            B.gmu[3 * src] = w.x;
+            B.gmu[3 * src + 1] = w.y;
+            B.gmu[3 * src + 2] = w.z;
+            if ((hd >> src) & 1u) {
+                const double m = d.mus[site];
+                B.gfo[src] = make_float4((float)(v.x * m), (float)(v.y * m), (float)(v.z * m), (float)m);
+                B.gfn[src] = make_float4((float)(w.x * m), (float)(w.y * m), (float)(w.z * m), (float)m);
+            }
+        } else if (pos) {
+            int64_t Y[3] = {X[0], X[1], X[2]};
+            if (rot) {
+                Y[0] = (int64_t)((uint64_t)c[0] + (uint64_t)__double2ll_rn(w.x * d.inv64d[0]));
+                Y[1] = (int64_t)((uint64_t)c[1] + (uint64_t)__double2ll_rn(w.y * d.inv64d[1]));
+                Y[2] = (int64_t)((uint64_t)c[2] + (uint64_t)__double2ll_rn(w.z * d.inv64d[2]));
+            }
+            if (trans)
+                for (int a = 0; a < 3; a++) Y[a] = (int64_t)((uint64_t)Y[a] + (uint64_t)tr.t[a]);
+            if (it == gs) {
+                if (explicit_ && d.expl_cm)
+                    for (int a = 0; a < 3; a++) Y[a] = d.expl_cm[a];
+                for (int a = 0; a < 3; a++) B.gcm[a] = Y[a];
+            } else {
+                if (explicit_)
+                    for (int a = 0; a < 3; a++) Y[a] = d.expl_pos[3 * it + a];
+                const int4 go = make_int4(hi32(X[0]), hi32(X[1]), hi32(X[2]), type | (has_dip ? 0x100 : 0));
+                const int4 gn = make_int4(hi32(Y[0]), hi32(Y[1]), hi32(Y[2]), type | (site << 8));
+                B.go[it] = go;
+                B.gn[it] = gn;
+                for (int a = 0; a < 3; a++) B.gX[3 * it + a] = Y[a];
+                const float3 o = make_float3((float)wsub(go.x, rf[0]) * s32.x, (float)wsub(go.y, rf[1]) * s32.y,
+                                             (float)wsub(go.z, rf[2]) * s32.z);
+                const float3 n = make_float3((float)wsub(gn.x, rf[0]) * s32.x, (float)wsub(gn.y, rf[1]) * s32.y,
+                                             (float)wsub(gn.z, rf[2]) * s32.z);
+                dlo = make_float4(o.x, o.y, o.z, dot3f(o, o));
+                dln = make_float4(n.x, n.y, n.z, dot3f(n, n));
+                B.dlo[it] = dlo;
+                B.dln[it] = dln;
+            }
+        }
     }
-    const int site = g * gs + lane;
-    const int64_t Xo[3] = {P[3 * site], P[3 * site + 1], P[3 * site + 2]};
-    int64_t Xn[3];
-    const D3 uo = {MU[3 * site], MU[3 * site + 1], MU[3 * site + 2]};
-    D3 un;
-    if (explicit_) {
-        for (int a = 0; a < 3; a++) Xn[a] = d.expl_pos[3 * lane + a];
-        un = d.expl_mu ? D3{d.expl_mu[3 * lane], d.expl_mu[3 * lane + 1], d.expl_mu[3 * lane + 2]} : uo;
-    } else {
-        move_point(Xo, Xn);
-        un = (tr.flags & 1) ? qrot(tr.qw, qv, uo) : uo;  // DipoleParticle::rotate (point.h:672-679)
+    // bounds of the offsets (non-negative floats order as their bit patterns)
+    auto wmax = [](float x) { return __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(x))); };
+    const float mx = wmax(fmaxf(fabsf(dlo.x), fabsf(dln.x))), my_ = wmax(fmaxf(fabsf(dlo.y), fabsf(dln.y)));
+    const float mz = wmax(fmaxf(fabsf(dlo.z), fabsf(dln.z))), mr = wmax(fmaxf(dlo.w, dln.w));
+    if (lane == 0) {
+        // the expanded r^2 loses (|D| / r)^2 in relative accuracy: a molecule
+        // longer than the cutoff tests every pair with direct distances
+        const float lim = (sqrtf(d.rc2near) + sqrtf(mr)) * 1.00001f;
+        const float hb = 2147483648.0f * 0.999998f;   // half box in high-word units, with a margin for rounding
+        *B.lim = make_float4(hb * s32.x - mx, hb * s32.y - my_, hb * s32.z - mz, mr <= d.rc2near ? lim * lim : 3.0e38f);
+        *B.ref = make_int4(rf[0], rf[1], rf[2], (int)hd);
+        *B.qmask = hq;
     }
-    const int type = d.pos4[site].w & 0xFF;
-    const bool has_dip = d.site_dip[site] >= 0;
-    const double m = d.mus[site];
-    B.go[lane] = make_int4(hi32(Xo[0]), hi32(Xo[1]), hi32(Xo[2]), type | (has_dip ? 0x100 : 0));
-    B.gn[lane] = make_int4(hi32(Xn[0]), hi32(Xn[1]), hi32(Xn[2]), type | (site << 8));
-    B.gfo[lane] = make_float4((float)(uo.x * m), (float)(uo.y * m), (float)(uo.z * m), (float)m);
-    B.gfn[lane] = make_float4((float)(un.x * m), (float)(un.y * m), (float)(un.z * m), (float)m);
-    B.gmu[3 * lane] = un.x;
-    B.gmu[3 * lane + 1] = un.y;
-    B.gmu[3 * lane + 2] = un.z;
-    for (int a = 0; a < 3; a++) B.gX[3 * lane + a] = Xn[a];
 }
 
 // ---------------------------------------------------------------- energy change
-// Warp-aggregated append of near pairs to the queue; a full queue makes the
-// lanes evaluate their pair in place (returned in `inplace`).
-__device__ __forceinline__ bool enqueue(const MolSmem &s, bool near, uint32_t code) {
-    const unsigned active = __activemask();
-    const unsigned m = __ballot_sync(active, near);
-    if (!m) return false;
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(m) - 1;
-    int base = 0;
-    if (lane == leader) base = atomicAdd(s.qcount, __popc(m));
-    base = __shfl_sync(active, base, leader);
-    if (!near) return false;
-    const int slot = base + __popc(m & ((1u << lane) - 1u));
-    if (slot < kQueueCap) {
-        s.queue[slot] = code;
-        return false;
+// LJ of the moved sites against one site per lane at displacement D from the
+// reference point, new minus old, any image (min(|dx|, L - |dx|)). With
+// y = r^-6 and c = sigma^6, u = 4eps (c^2 y^2 - c y), so u_n - u_o =
+// 4eps c dy (c (y_n + y_o) - 1), dy = y_n - y_o: uniform tables sum b1 = sum dy
+// and b2 = sum dy (y_n + y_o) and scale at the end; else b1 sums the energies.
+// Pairs within rc2near are left out and their bits returned.
+struct MolView {   // the same in every thread of a warp
+    float3 s32, L, half;   // Angstrom per high-word unit, box, half box less max |offset|
+    int4 ref;
+    float far2;            // sites beyond this squared distance from ref have no near pair
+};
+__device__ __forceinline__ MolView mol_view(const GroupBuf &B, float3 s32, float3 L) {
+    const float4 lim = *B.lim;
+    return MolView{s32, L, make_float3(lim.x, lim.y, lim.z), *B.ref, lim.w};
+}
+__device__ __forceinline__ float3 mol_disp(int4 p, const MolView &v) {
+    return make_float3((float)wsub(p.x, v.ref.x) * v.s32.x, (float)wsub(p.y, v.ref.y) * v.s32.y,
+                       (float)wsub(p.z, v.ref.z) * v.s32.z);
+}
+__device__ __forceinline__ int mol_outside(float3 D, const MolView &v) {   // axes on which some pair may change image
+    return (fabsf(D.x) > v.half.x ? 1 : 0) + (fabsf(D.y) > v.half.y ? 1 : 0) + (fabsf(D.z) > v.half.z ? 1 : 0);
+}
+template <bool UNI>
+__device__ __forceinline__ void mol_lj_add(const MolDesc &d, int ti, int tj, float yo, float yn, float &b1, float &b2) {
+    const float dy = yn - yo, sy = yn + yo;
+    if (UNI) {
+        b1 += dy;
+        b2 = fmaf(dy, sy, b2);
+    } else {
+        const int t = ti * d.nt + tj;
+        const float s2 = d.s2[t], c = s2 * s2 * s2;
+        b1 = fmaf(d.eps4[t] * c * dy, fmaf(c, sy, -1.0f), b1);
     }
-    return true;
+}
+template <bool UNI>
+__device__ __forceinline__ uint32_t mol_lj_image(const MolDesc &d, const GroupBuf &B, const MolView &v, float3 D,
+                                                 int tj, float &b1, float &b2) {
+    uint32_t near = 0u;
+    const int gs = d.gs;
+    const float rc2near = d.rc2near;
+    auto r2_of = [&](float4 o) {
+        const float x = fabsf(D.x - o.x), y = fabsf(D.y - o.y), z = fabsf(D.z - o.z);
+        const float mx = fminf(x, v.L.x - x), my = fminf(y, v.L.y - y), mz = fminf(z, v.L.z - z);
+        return fmaf(mx, mx, fmaf(my, my, mz * mz));
+    };
+#pragma unroll 4
+    for (int i = 0; i < gs; i++) {
+        const float r2o = r2_of(B.dlo[i]), r2n = r2_of(B.dln[i]);
+        const float io = rcp_approx(r2o), in_ = rcp_approx(r2n);
+        const bool nr = fminf(r2o, r2n) < rc2near;
+        near |= nr ? 1u << i : 0u;
+        const float yo = nr ? 0.0f : io * io * io, yn = nr ? 0.0f : in_ * in_ * in_;
+        mol_lj_add<UNI>(d, UNI ? 0 : B.go[i].w & 0xFF, tj, yo, yn, b1, b2);
+    }
+    return near;
+}
+// The same for kMolPerLane sites per lane that need no image: r^2 = |D|^2 +
+// |delta|^2 - 2 D.delta from D2 = -2 D and A = |D|^2. A pair of distances takes
+// 18 issue slots and two MUFU (against about 170 when every pair converted
+// six integer differences); four sites share the two 16-byte loads of an
+// offset pair, whose 512-byte broadcasts would otherwise fill the
+// shared-memory port (8 of every 20 cycles per warp and SM quarter).
+template <bool UNI>
+__device__ __forceinline__ void mol_lj_far(const MolDesc &d, const GroupBuf &B, const float3 (&D2)[kMolPerLane],
+                                           const float (&A)[kMolPerLane], const int (&tj)[kMolPerLane], float &b1,
+                                           float &b2) {
+    const int gs = d.gs;
+#pragma unroll 2
+    for (int i = 0; i < gs; i++) {
+        const float4 o = B.dlo[i], n = B.dln[i];
+        const int ti = UNI ? 0 : B.go[i].w & 0xFF;
+#pragma unroll
+        for (int u = 0; u < kMolPerLane; u++) {
+            const float io = rcp_approx(fmaf(o.x, D2[u].x, fmaf(o.y, D2[u].y, fmaf(o.z, D2[u].z, A[u] + o.w))));
+            const float in_ = rcp_approx(fmaf(n.x, D2[u].x, fmaf(n.y, D2[u].y, fmaf(n.z, D2[u].z, A[u] + n.w))));
+            mol_lj_add<UNI>(d, ti, tj[u], io * io * io, in_ * in_ * in_, b1, b2);
+        }
+    }
 }
 
-// This CTA's part of dU for the trial in buffer B. Pair loops use threads
-// [0, nwork); the queue is drained by all threads.
+// The same for one far site per lane whose image may change along one axis:
+// the nearer of its two images along that axis, |D - delta|^2 and
+// |D' - delta|^2 with D' = D -+ L, each expanded (28 issue slots per pair
+// against 43 of the general form above).
+template <bool UNI>
+__device__ __forceinline__ void mol_lj_edge(const MolDesc &d, const GroupBuf &B, const MolView &v, float3 D, int tj,
+                                            float &b1, float &b2) {
+    float3 E = D;
+    if (fabsf(D.x) > v.half.x) E.x = D.x - copysignf(v.L.x, D.x);
+    else if (fabsf(D.y) > v.half.y) E.y = D.y - copysignf(v.L.y, D.y);
+    else E.z = D.z - copysignf(v.L.z, D.z);
+    const float A = dot3f(D, D), AE = dot3f(E, E);
+    const float3 D2 = make_float3(-2.0f * D.x, -2.0f * D.y, -2.0f * D.z);
+    const float3 E2 = make_float3(-2.0f * E.x, -2.0f * E.y, -2.0f * E.z);
+    auto r2_of = [&](float4 o) {
+        return fminf(fmaf(o.x, D2.x, fmaf(o.y, D2.y, fmaf(o.z, D2.z, A + o.w))),
+                     fmaf(o.x, E2.x, fmaf(o.y, E2.y, fmaf(o.z, E2.z, AE + o.w))));
+    };
+    const int gs = d.gs;
+#pragma unroll 4
+    for (int i = 0; i < gs; i++) {
+        const float io = rcp_approx(r2_of(B.dlo[i])), in_ = rcp_approx(r2_of(B.dln[i]));
+        mol_lj_add<UNI>(d, UNI ? 0 : B.go[i].w & 0xFF, tj, io * io * io, in_ * in_ * in_, b1, b2);
+    }
+}
+
+// W of IonDipole without its prefactor: (f_n . r_n) / r_n^3 - (f_o . r_o) / r_o^3.
+__device__ __forceinline__ float ion_dipole_diff(float3 fo, float3 ro, float3 fn, float3 rn) {
+    const float ro2 = dot3f(ro, ro), rn2 = dot3f(rn, rn);
+    const float io = rsqrtf(ro2), in_ = rsqrtf(rn2);
+    return dot3f(fn, rn) * in_ * in_ * in_ - dot3f(fo, ro) * io * io * io;
+}
+__device__ __forceinline__ float3 xyz(float4 v) { return make_float3(v.x, v.y, v.z); }
+__device__ __forceinline__ float3 sub3(float4 a, float3 b) { return make_float3(a.x - b.x, a.y - b.y, a.z - b.z); }
+// W2 of IonDipole(a = i, b = j) over the moved dipoles in mask m, with lbq =
+// lB q_j: -lB q_j (mu_i . r) / r^3, r = r_i - r_j (exact image).
+__device__ __forceinline__ float mol_w2_exact(const GroupBuf &B, uint32_t m, int4 pj, float lbq, float3 s32) {
+    float w = 0.0f;
+    for (; m; m &= m - 1) {
+        const int i = __ffs(m) - 1;
+        w -= lbq * ion_dipole_diff(xyz(B.gfo[i]), diff32(B.go[i], pj, s32), xyz(B.gfn[i]), diff32(B.gn[i], pj, s32));
+    }
+    return w;
+}
+
+// A queued near pair: moved site << 24 | dipole flag (0x800000) | slice index.
 template <bool SLICE_SMEM>
-__device__ float mol_partial_loops(const MolDesc &d, const MolSmem &s, const GroupBuf &B, int g, int j0, int ns,
-                                   int nd, int nwork) {
-    const int tid = threadIdx.x, gs = d.gs;
+__device__ __noinline__ float mol_near_pair(const MolDesc &d, const MolSmem &s, const GroupBuf &B, uint32_t c, int j0) {
+    const int i = (int)((c >> 24) & 0x7F), idx = (int)(c & 0x7FFFFF);
+    if (c & 0x800000u) return near_pair_b(B.go[i], B.gn[i], B.gfo[i], B.gfn[i], s.sdpos[idx], s.sdip[idx], d);
+    return near_pair_a(B.go[i], B.gn[i], B.gfo[i], B.gfn[i], SLICE_SMEM ? s.spos[idx] : d.pos4[j0 + idx], d);
+}
+// The CTA's queued near pairs, 32 of one warp's queue at a time over all warps
+// (chunk c of the queues laid end to end goes to warp c % kMolWarps); each
+// result replaces its pair in the queue. Between block barriers.
+template <bool SLICE_SMEM>
+__device__ __forceinline__ void mol_near_pairs(const MolDesc &d, const MolSmem &s, int parts, int j0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int mine = lane < kMolWarps ? s.npair[lane] : 0, nch = (mine + 31) >> 5;
+    int end = nch;   // inclusive prefix sum of the chunks
+#pragma unroll
+    for (int o = 1; o < kMolWarps; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += x;
+    }
+    const int total = __shfl_sync(0xffffffffu, end, kMolWarps - 1);
+    for (int c = warp; c < total; c += kMolWarps) {
+        const int w = __popc(__ballot_sync(0xffffffffu, lane < kMolWarps && end <= c));   // the queue's warp
+        const int k = (c - __shfl_sync(0xffffffffu, end - nch, w)) * 32 + lane;
+        if (k < __shfl_sync(0xffffffffu, mine, w)) {
+            uint32_t *q = s.queue + w * kMolQueue + 2 * kMolSiteQueue + k;
+            *q = __float_as_uint(mol_near_pair<SLICE_SMEM>(d, s, mol_group(s, d.gs, w / parts), *q, j0));
+        }
+    }
+}
+
+// One warp's part of dU for trial m of the group (molecule g) over this CTA's
+// slice (part `part` of `parts`): the site groups and dipole chunks part, part
+// + parts, ... Sites beyond reach of the cutoff that need no image go through
+// mol_lj_far as they come; those that may change image and those that may be
+// near are collected in the warp's queues and taken 32 at a time. The near
+// pairs stay in the warp's pair queue (their number to npair): all warps of the
+// CTA share them out afterwards (mol_near_pairs), since a close molecule puts
+// its 400 pairs on one warp. Everything is in a fixed order, and each kind of
+// work has one place in the loop (the code stays within the instruction
+// cache). All lanes call it; the lane's part of the sum is returned (df).
+template <bool SLICE_SMEM, bool UNI>
+__device__ __noinline__ df mol_base(const MolDesc &d, const MolSmem &sm, int m, int g, int j0, int ns, int nd,
+                                    float3 s32, float3 L, int part, int parts) {
+    const MolSmem s = sm;
+    const int lane = threadIdx.x & 31, gs = d.gs;
+    const uint32_t full = 0xffffffffu, below = (1u << lane) - 1u;
+    const GroupBuf B = mol_group(s, gs, m);
+    const MolView v = mol_view(B, s32, L);
     const int g_lo = g * gs, g_hi = g_lo + gs;
-    const float3 sc9 = make_float3(d.sc9[0], d.sc9[1], d.sc9[2]);
-    const float3 s32 = make_float3(d.s32[0], d.s32[1], d.s32[2]);
-    const float rc2near = d.rc2near, lB = d.lB;
-    const int nt = d.nt;
-    const bool uni = d.uniform_lj != 0;
-    const float s2u = d.s2[0], e4u = d.eps4[0];
-    float acc = 0.0f;
-    if (tid >= nwork) return 0.0f;
-    // loop A: slice sites j (one per thread) against every moved site i;
-    // whole warps iterate together so the queue appends stay warp-wide
-    for (int jb = tid - (tid & 31); jb < ns; jb += nwork) {
-        const int jj = jb + (tid & 31);
-        const int j = j0 + jj;
-        const bool valid = jj < ns && !(j >= g_lo && j < g_hi);
-        const int4 pj = SLICE_SMEM ? s.spos[min(jj, ns - 1)] : d.pos4[j0 + min(jj, ns - 1)];
-        const int tj = pj.w & 0xFF;
-        const float qj = d.qtype[tj];
-#pragma unroll 2
-        for (int i = 0; i < gs; i++) {
-            const int4 po = B.go[i], pn = B.gn[i];
-            const int t = (po.w & 0xFF) * nt + tj;
-            const float s2 = uni ? s2u : d.s2[t], e4 = uni ? e4u : d.eps4[t];
-            const float r2o = far_r2(po, pj, sc9), r2n = far_r2(pn, pj, sc9);
-            const bool near = valid && ((r2o < rc2near) | (r2n < rc2near));
-            if (enqueue(s, near, ((uint32_t)i << 24) | (uint32_t)jj))
-                acc += near_pair_a(po, pn, B.gfo[i], B.gfn[i], pj, d);
-            if (valid && !near) {
-                acc += lj_r2(r2n, s2, e4) - lj_r2(r2o, s2, e4);
-                if ((po.w & 0x100) && qj != 0.0f) {
-                    // W2 of IonDipole(a = i, b = j): -lB q_j (mu_i . r) / r^3
-                    const float3 ro = diff32(po, pj, s32), rn = diff32(pn, pj, s32);
-                    const float4 fo = B.gfo[i], fn = B.gfn[i];
-                    const float ro2 = dot3f(ro, ro), rn2 = dot3f(rn, rn);
-                    const float io = rsqrtf(ro2), in_ = rsqrtf(rn2);
-                    const float w = dot3f(make_float3(fn.x, fn.y, fn.z), rn) * in_ * in_ * in_ -
-                                    dot3f(make_float3(fo.x, fo.y, fo.z), ro) * io * io * io;
-                    acc -= lB * qj * w;
+    const uint32_t dips = (uint32_t)v.ref.w;
+    uint32_t *const bq = s.queue + (threadIdx.x >> 5) * kMolQueue, *const nq = bq + kMolSiteQueue,
+             *const pq = nq + kMolSiteQueue;
+    int nb = 0, nn = 0, np = 0;
+    float b1 = 0.0f, b2 = 0.0f;
+    df acc = {0.0f, 0.0f};
+    auto site = [&](int jj) { return SLICE_SMEM ? s.spos[jj] : d.pos4[j0 + jj]; };
+    auto push = [&](uint32_t *q, int &cnt, bool f, uint32_t val) {
+        const uint32_t b = __ballot_sync(full, f);
+        if (f) q[cnt + __popc(b & below)] = val;
+        cnt += __popc(b);
+    };
+    auto drop = [&](uint32_t *q, int &cnt) {   // the first 32 entries are done: the rest moves up (a lane
+        cnt = max(cnt - 32, 0);                 // writes only what it read itself)
+        for (int e = lane; e < cnt; e += 32) q[e] = q[32 + e];
+        __syncwarp();
+    };
+    const int gsites = 32 * kMolPerLane, nsg = (ns + gsites - 1) / gsites, ndg = (nd + 31) >> 5;
+    for (int it = part; it < nsg + ndg; it += parts) {
+        const bool last = it + parts >= nsg + ndg;   // this warp's last turn: the queues are emptied
+        uint32_t near = 0u, code = 0u;
+        if (it < nsg) {
+            float3 D2[kMolPerLane];
+            float A[kMolPerLane], lbq[kMolPerLane];
+            int tj[kMolPerLane];
+            bool any = false;
+#pragma unroll
+            for (int u = 0; u < kMolPerLane; u++) {
+                const int jj = it * gsites + 32 * u + lane, j = j0 + jj;
+                const bool in = jj < ns && !(j >= g_lo && j < g_hi);
+                const int4 pj = site(min(jj, ns - 1));
+                tj[u] = pj.w & 0xFF;
+                const float3 D = mol_disp(pj, v);
+                A[u] = dot3f(D, D);
+                const int axes = mol_outside(D, v);
+                const bool nr = in && (A[u] <= v.far2 || axes > 1);   // near, or a rare image along several axes
+                const bool edge = in && !nr && axes == 1;
+                const bool ok = in && !nr && !edge;
+                if (__any_sync(full, nr || edge)) {
+                    push(nq, nn, nr, (uint32_t)jj);
+                    push(bq, nb, edge, (uint32_t)jj);
+                }
+                // a site taken elsewhere sits so far away that its terms vanish
+                D2[u] = ok ? make_float3(-2.0f * D.x, -2.0f * D.y, -2.0f * D.z) : make_float3(-2.0e15f, 0.0f, 0.0f);
+                A[u] = ok ? A[u] : 1.0e30f;
+                lbq[u] = ok ? s.lbq[tj[u]] : 0.0f;
+                any |= lbq[u] != 0.0f;
+            }
+            mol_lj_far<UNI>(d, B, D2, A, tj, b1, b2);
+            if (dips != 0u && __any_sync(full, any)) {
+                float w = 0.0f;
+                for (uint32_t q = dips; q; q &= q - 1) {
+                    const int i = __ffs(q) - 1;
+                    const float4 o = B.dlo[i], n = B.dln[i];
+                    const float3 fo = xyz(B.gfo[i]), fn = xyz(B.gfn[i]);
+#pragma unroll
+                    for (int u = 0; u < kMolPerLane; u++) {
+                        const float3 D = make_float3(-0.5f * D2[u].x, -0.5f * D2[u].y, -0.5f * D2[u].z);
+                        w = fmaf(-lbq[u], ion_dipole_diff(fo, sub3(o, D), fn, sub3(n, D)), w);
+                    }
+                }
+                acc = df_add_f(acc, w);
+            }
+        } else {
+            // dipoles of the slice against the moved charges: W1 of IonDipole(a = i,
+            // b = k): lB q_i (mu_k . r) / r^3 (dipole-dipole is 0 beyond rc: near pairs)
+            const int kk = (it - nsg) * 32 + lane, kc = min(kk, nd - 1);
+            const int4 pk = s.sdpos[kc];
+            const float3 f = xyz(s.sdip[kc]);
+            const int ksite = pk.w >> 8;
+            const bool in = kk < nd && !(ksite >= g_lo && ksite < g_hi);
+            const float3 D = mol_disp(pk, v);
+            float w = 0.0f;
+            if (__any_sync(full, in && dot3f(D, D) <= v.far2)) {
+                for (int i = 0; i < gs; i++) {
+                    const float3 ro = diff32(B.go[i], pk, s32), rn = diff32(B.gn[i], pk, s32);
+                    const bool nr = in && fminf(dot3f(ro, ro), dot3f(rn, rn)) < d.rc2near;
+                    near |= nr ? 1u << i : 0u;
+                    const float q = s.lbq[B.go[i].w & 0xFF];
+                    if (!nr && q != 0.0f) w = fmaf(q, ion_dipole_diff(f, ro, f, rn), w);
+                }
+            } else {
+                const bool image = __any_sync(full, in && mol_outside(D, v) != 0);
+                for (uint32_t q = *B.qmask; q; q &= q - 1) {
+                    const int i = __ffs(q) - 1;
+                    const int4 po = B.go[i];
+                    float3 ro = sub3(B.dlo[i], D), rn = sub3(B.dln[i], D);
+                    if (image) {
+                        ro = diff32(po, pk, s32);
+                        rn = diff32(B.gn[i], pk, s32);
+                    }
+                    w = fmaf(s.lbq[po.w & 0xFF], ion_dipole_diff(f, ro, f, rn), w);
                 }
             }
+            if (in) acc = df_add_f(acc, w);
+            code = 0x800000u | (uint32_t)kk;
         }
-    }
-    // loop B: (dipole k of this slice, moved site i) items spread over threads
-    const int nitems = nd * gs;
-    for (int eb = tid - (tid & 31); eb < nitems; eb += nwork) {
-        const int e = eb + (tid & 31);
-        const int kk = min(e, nitems - 1) / gs, i = min(e, nitems - 1) - kk * gs;
-        const int4 pk = s.sdpos[kk];
-        const int ksite = pk.w >> 8;
-        const bool valid = e < nitems && !(ksite >= g_lo && ksite < g_hi);
-        const int4 po = B.go[i], pn = B.gn[i];
-        const float3 ro = diff32(po, pk, s32), rn = diff32(pn, pk, s32);
-        const float ro2 = dot3f(ro, ro), rn2 = dot3f(rn, rn);
-        const bool near = valid && ((ro2 < rc2near) | (rn2 < rc2near));
-        if (enqueue(s, near, 0x800000u | ((uint32_t)i << 24) | (uint32_t)kk))
-            acc += near_pair_b(po, pn, B.gfo[i], B.gfn[i], pk, s.sdip[kk], d);
-        if (valid && !near) {
-            const float qi = d.qtype[po.w & 0xFF];
-            if (qi != 0.0f) {
-                // W1 of IonDipole(a = i, b = k): lB q_i (mu_k . r) / r^3 (dipole-dipole is 0 beyond rc)
-                const float4 vk = s.sdip[kk];
-                const float3 v = make_float3(vk.x, vk.y, vk.z);
-                const float io = rsqrtf(ro2), in_ = rsqrtf(rn2);
-                acc += lB * qi * (dot3f(v, rn) * in_ * in_ * in_ - dot3f(v, ro) * io * io * io);
+        __syncwarp();
+        const int lim = last ? 1 : 32;
+        while (true) {
+            while (__any_sync(full, near != 0u)) {   // near pairs of this turn, one per lane at a time
+                push(pq, np, near != 0u, ((uint32_t)(__ffs(near) - 1) << 24) | code);
+                near &= near - 1;
+                if (np > kMolPairQueue - 32) {   // no room for another turn: the last 32 now
+                    __syncwarp();
+                    np -= 32;
+                    acc = df_add_f(acc, mol_near_pair<SLICE_SMEM>(d, s, B, pq[np + lane], j0));
+                    __syncwarp();
+                }
             }
+            if (nn < lim && nb < lim) break;
+            // up to 32 sites: near ones first (near stays 0 for the others)
+            const bool nearq = nn >= lim;
+            uint32_t *q = nearq ? nq : bq;
+            const int cnt = nearq ? nn : nb;
+            const int jj = (int)q[min(lane, cnt - 1)];
+            const int4 pj = site(jj);
+            float c1 = 0.0f, c2 = 0.0f;
+            if (nearq) near = mol_lj_image<UNI>(d, B, v, mol_disp(pj, v), pj.w & 0xFF, c1, c2);
+            else mol_lj_edge<UNI>(d, B, v, mol_disp(pj, v), pj.w & 0xFF, c1, c2);
+            if (lane < cnt) {
+                b1 += c1;
+                b2 += c2;
+                const float lbq = s.lbq[pj.w & 0xFF];
+                if (lbq != 0.0f) acc = df_add_f(acc, mol_w2_exact(B, dips & ~near, pj, lbq, s32));
+            } else {
+                near = 0u;
+            }
+            code = (uint32_t)jj;
+            __syncwarp();
+            if (nearq) drop(nq, nn);
+            else drop(bq, nb);
         }
     }
-    return acc;
+    if (lane == 0) s.npair[threadIdx.x >> 5] = np;
+    if (UNI) {
+        const float c = d.s2[0] * d.s2[0] * d.s2[0];
+        return df_add_f(acc, d.eps4[0] * c * fmaf(c, b2, -b1));
+    }
+    return df_add_f(acc, b1);
 }
 
-template <bool SLICE_SMEM>
-__device__ float mol_partial_queue(const MolDesc &d, const MolSmem &s, const GroupBuf &B, int j0) {
-    const int nq = min(*s.qcount, kQueueCap);
-    float acc = 0.0f;
-    for (int e = threadIdx.x; e < nq; e += blockDim.x) {
-        const uint32_t q = s.queue[e];
-        const int i = (int)((q >> 24) & 0x7F);
-        const int idx = (int)(q & 0x7FFFFF);
-        if (q & 0x800000u) {
-            acc += near_pair_b(B.go[i], B.gn[i], B.gfo[i], B.gfn[i], s.sdpos[idx], s.sdip[idx], d);
+// c(a, m): how much dU of trial m (buffer Bm) changes when trial a (buffer Ba,
+// another molecule) is accepted: m's energy change against a's sites at their
+// new positions minus that at their old ones. One warp; lanes over a's sites.
+template <bool UNI>
+__device__ __noinline__ df mol_correction(const MolDesc &d, const MolSmem &sm, int a, int m, float3 s32, float3 L) {
+    const MolSmem s = sm;
+    const int lane = threadIdx.x & 31, gs = d.gs;
+    const GroupBuf Ba = mol_group(s, gs, a), Bm = mol_group(s, gs, m);
+    const uint32_t full = 0xffffffffu;
+    const MolView v = mol_view(Bm, s32, L);
+    const bool in = lane < gs;
+    const int4 pn = Ba.gn[min(lane, gs - 1)], po = Ba.go[min(lane, gs - 1)];
+    const float3 Dn = mol_disp(pn, v), Do = mol_disp(po, v);
+    const uint32_t dm = (uint32_t)v.ref.w, da = (uint32_t)Ba.ref->w, qm = *Bm.qmask;
+    df acc = {0.0f, 0.0f};
+    if (__any_sync(full, in && (dot3f(Dn, Dn) <= v.far2 || dot3f(Do, Do) <= v.far2))) {
+        // close molecules: every site pair in the near form
+        for (int e = lane; e < gs * gs; e += 32) {
+            const int i = e / gs, j = e - i * gs;
+            acc = df_add_f(acc, near_pair_a(Bm.go[i], Bm.gn[i], Bm.gfo[i], Bm.gfn[i], Ba.gn[j], d));
+            acc = df_add_f(acc, -near_pair_a(Bm.go[i], Bm.gn[i], Bm.gfo[i], Bm.gfn[i], Ba.go[j], d));
+            if ((da >> j) & 1u) {
+                acc = df_add_f(acc, near_pair_b(Bm.go[i], Bm.gn[i], Bm.gfo[i], Bm.gfn[i], Ba.gn[j], Ba.gfn[j], d));
+                acc = df_add_f(acc, -near_pair_b(Bm.go[i], Bm.gn[i], Bm.gfo[i], Bm.gfn[i], Ba.go[j], Ba.gfo[j], d));
+            }
+        }
+        return warp_sum_df(acc);
+    }
+    const int tj = po.w & 0xFF;
+    float n1 = 0.0f, n2 = 0.0f, o1 = 0.0f, o2 = 0.0f;
+    auto y_of = [&](float3 D, float4 o) {   // r^-6, any image
+        const float x = fabsf(D.x - o.x), y = fabsf(D.y - o.y), z = fabsf(D.z - o.z);
+        const float mx = fminf(x, L.x - x), my = fminf(y, L.y - y), mz = fminf(z, L.z - z);
+        const float i = rcp_approx(fmaf(mx, mx, fmaf(my, my, mz * mz)));
+        return i * i * i;
+    };
+#pragma unroll 4
+    for (int i = 0; i < gs; i++) {
+        const float4 o = Bm.dlo[i], n = Bm.dln[i];
+        const int ti = UNI ? 0 : Bm.go[i].w & 0xFF;
+        mol_lj_add<UNI>(d, ti, tj, y_of(Dn, o), y_of(Dn, n), n1, n2);
+        mol_lj_add<UNI>(d, ti, tj, y_of(Do, o), y_of(Do, n), o1, o2);
+    }
+    if (in) {
+        if (UNI) {
+            const float c = d.s2[0] * d.s2[0] * d.s2[0];
+            acc = df_add_f(acc, d.eps4[0] * c * fmaf(c, n2 - o2, o1 - n1));
         } else {
-            const int4 pj = SLICE_SMEM ? s.spos[idx] : d.pos4[j0 + idx];
-            acc += near_pair_a(B.go[i], B.gn[i], B.gfo[i], B.gfn[i], pj, d);
+            acc = df_add_f(acc, n1 - o1);
+        }
+        // m's dipoles with a's charges, a's dipoles with m's charges
+        const float lbq = s.lbq[tj];
+        if (lbq != 0.0f)
+            acc = df_add_f(acc, mol_w2_exact(Bm, dm, pn, lbq, s32) - mol_w2_exact(Bm, dm, po, lbq, s32));
+        if ((da >> lane) & 1u) {
+            const float3 fn = xyz(Ba.gfn[lane]), fo = xyz(Ba.gfo[lane]);
+            float w = 0.0f;
+            for (uint32_t m = qm; m; m &= m - 1) {
+                const int i = __ffs(m) - 1;
+                w = fmaf(s.lbq[Bm.go[i].w & 0xFF],
+                         ion_dipole_diff(fn, diff32(Bm.go[i], pn, s32), fn, diff32(Bm.gn[i], pn, s32)) -
+                             ion_dipole_diff(fo, diff32(Bm.go[i], po, s32), fo, diff32(Bm.gn[i], po, s32)),
+                         w);
+            }
+            acc = df_add_f(acc, w);
         }
     }
-    return acc;
+    return warp_sum_df(acc);
 }
 
 // ---------------------------------------------------------------- the sweep
 // One cluster of C CTAs per system (blockIdx.x / C). EVAL: evaluate trial 0
-// only, write its dU to eval_du, decide and commit nothing. The last warp
-// prepares the next trial's coordinates while the others sum pairs; the
-// prepared buffer is discarded when an accepted trial moved the same molecule.
+// only, write its dU to eval_du, decide and commit nothing. Groups of up to
+// `ahead` trials; a group of fewer trials than warps splits each trial's slice
+// over several warps.
 template <bool SLICE_SMEM, bool CLUSTER, bool EVAL>
-__global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc *__restrict__ descs) {
+__global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc *__restrict__ descs, int ahead,
+                                                                  int64_t quantum) {
     extern __shared__ __align__(16) unsigned char mol_smem_raw[];
     const int C = CLUSTER ? (int)descs[0].C : 1;
     const int sys = blockIdx.x / C;
-    // launch-shape check: partial sums are read from C CTAs of this cluster
+    // launch-shape check: partial sums come from C CTAs of this cluster
     if (CLUSTER && (int)cluster_size() != C) {
         if (threadIdx.x == 0) atomicOr(&descs[sys].sc->error, kMolErrLaunch);
         return;
     }
     const int rank = CLUSTER ? (int)cluster_rank() : 0;
     const MolDesc &d = descs[sys];
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int nwork = (int)blockDim.x - 32;           // threads on the pair loops
-    const bool setup_warp = tid >= nwork;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int ns_full = (d.N + C - 1) / C, nd_full = (d.D + C - 1) / C;
     const int j0 = min(rank * ns_full, d.N), j1 = min(j0 + ns_full, d.N), ns = j1 - j0;
     const int k0 = min(rank * nd_full, d.D), k1 = min(k0 + nd_full, d.D), nd = k1 - k0;
-    MolSmem s = mol_carve(mol_smem_raw, ns_full, nd_full, d.gs, SLICE_SMEM);
+    MolSmem s = mol_carve(mol_smem_raw, ns_full, nd_full, d.gs, SLICE_SMEM, ahead);
     if (SLICE_SMEM)
         for (int jj = tid; jj < ns; jj += blockDim.x) s.spos[jj] = d.pos4[j0 + jj];
     for (int kk = tid; kk < nd; kk += blockDim.x) {
         s.sdip[kk] = d.dip4[k0 + kk];
         s.sdpos[kk] = d.dip_pos4[k0 + kk];
     }
+    if (tid < 16) s.lbq[tid] = tid < d.nt ? d.lB * d.qtype[tid] : 0.0f;
     int64_t cursor = EVAL ? 0 : d.sc->cursor;
-    const int64_t n = EVAL ? 1 : d.sc->n_trials;
+    const int64_t n = EVAL ? 1 : min(d.sc->n_trials, cursor + quantum);   // at most quantum trials of the stream
     df usum = {d.sc->u_hi, d.sc->u_lo};
     df utot = {d.sc->utot_hi, d.sc->utot_lo};
     int64_t nacc = d.sc->n_accepted;
-    int err = 0;
-    if (tid == 0) {
-        s.part[0] = s.part[1] = make_float2(0.0f, 0.0f);
-        s.flag[0] = s.flag[1] = 0;
-    }
-    if (cursor < n && setup_warp) setup_trial(d.trials[cursor], d, s.buf[cursor & 1], rank, lane);
-    if (CLUSTER) cluster_barrier();
-    else __syncthreads();
-    for (; cursor < n; cursor++) {
-        const int b = (int)(cursor & 1);
-        const MolTrial tr = d.trials[cursor];
-        if (s.flag[1]) {   // the prepared buffer is stale (same molecule, accepted)
-            __syncthreads();
-            if (setup_warp) setup_trial(tr, d, s.buf[b], rank, lane);
-            if (tid == 0) s.flag[1] = 0;
+    const bool uni = d.uniform_lj != 0;
+    const float3 s32 = make_float3(d.s32[0], d.s32[1], d.s32[2]);
+    const float3 L = make_float3(s32.x * 4294967296.0f, s32.y * 4294967296.0f, s32.z * 4294967296.0f);
+    int err = 0, buf = 0;
+    if (CLUSTER) cluster_barrier();   // every CTA of the cluster runs before any remote store
+    for (; cursor < n; buf ^= 1) {
+        const int ng = (int)(n - cursor < (int64_t)ahead ? n - cursor : (int64_t)ahead);
+        __syncthreads();   // the previous group's commits are in place
+        for (int m = warp; m < ng; m += kMolWarps)
+            setup_trial(d.trials[cursor + m], d, mol_group(s, d.gs, m), rank);
+        __syncthreads();
+        // ---- base sums: warp w takes part w % parts of trial w / parts
+        const int parts = kMolWarps / ng, tm = warp / parts;
+        float2 *const xpart = s.part + buf * kMaxCluster * kMolWarps, *const xcorr = s.corr + buf * kMolAhead * kMolAhead;
+        df v = {0.0f, 0.0f};
+        if (tm < ng) {
+            const int g = d.trials[cursor + tm].g;
+            v = uni ? mol_base<SLICE_SMEM, true>(d, s, tm, g, j0, ns, nd, s32, L, warp - tm * parts, parts)
+                    : mol_base<SLICE_SMEM, false>(d, s, tm, g, j0, ns, nd, s32, L, warp - tm * parts, parts);
+        } else if (lane == 0) {
+            s.npair[warp] = 0;
         }
-        if (tid == 0) *s.qcount = 0;
+        __syncthreads();   // the near pairs are queued
+        mol_near_pairs<SLICE_SMEM>(d, s, parts, j0);
         __syncthreads();
-        float part;
-        if (!setup_warp) {
-            part = mol_partial_loops<SLICE_SMEM>(d, s, s.buf[b], tr.g, j0, ns, nd, nwork);
-        } else {
-            part = 0.0f;
-            if (!EVAL && cursor + 1 < n) setup_trial(d.trials[cursor + 1], d, s.buf[b ^ 1], rank, lane);
-        }
-        __syncthreads();
-        part += mol_partial_queue<SLICE_SMEM>(d, s, s.buf[b], j0);
-        df pd = warp_sum_df(df{part, 0.0f});
-        if (lane == 0) s.red[tid >> 5] = make_float2(pd.hi, pd.lo);
-        __syncthreads();
-        const int slot = b;
-        if (tid < 32) {
-            df v = {0.0f, 0.0f};
-            if (tid < (int)(blockDim.x >> 5)) v = df{s.red[tid].x, s.red[tid].y};
+        if (tm < ng) {
+            const float *res = reinterpret_cast<const float *>(s.queue + warp * kMolQueue + 2 * kMolSiteQueue);
+            for (int k = lane; k < s.npair[warp]; k += 32) v = df_add_f(v, res[k]);
             v = warp_sum_df(v);
-            if (tid == 0) s.part[slot] = make_float2(v.hi, v.lo);
+            v.hi = __shfl_sync(0xffffffffu, v.hi, 0);   // one value for every CTA: they must decide alike
+            v.lo = __shfl_sync(0xffffffffu, v.lo, 0);
+            if (CLUSTER) {
+                if (lane < C) st_cluster_f2(&xpart[rank * kMolWarps + warp], (unsigned)lane, make_float2(v.hi, v.lo));
+            } else if (lane == 0) {
+                xpart[warp] = make_float2(v.hi, v.lo);
+            }
         }
+        // ---- corrections c(a, m), a < m, over the cluster's warps
+        if (!EVAL)
+            for (int e = rank * kMolWarps + warp, m = 1, lo = 0; e < ng * (ng - 1) / 2; e += C * kMolWarps) {
+                while (e >= lo + m) lo += m++;   // pair e of the triangle: trial m, a = e - m (m - 1) / 2
+                const int a = e - lo;
+                if (d.trials[cursor + a].g == d.trials[cursor + m].g) continue;
+                df c = uni ? mol_correction<true>(d, s, a, m, s32, L) : mol_correction<false>(d, s, a, m, s32, L);
+                c.hi = __shfl_sync(0xffffffffu, c.hi, 0);
+                c.lo = __shfl_sync(0xffffffffu, c.lo, 0);
+                if (CLUSTER) {
+                    if (lane < C) st_cluster_f2(&xcorr[a * kMolAhead + m], (unsigned)lane, make_float2(c.hi, c.lo));
+                } else if (lane == 0) {
+                    xcorr[a * kMolAhead + m] = make_float2(c.hi, c.lo);
+                }
+            }
         if (CLUSTER) cluster_barrier();
         else __syncthreads();
-        if (tid < 32) {
-            df v = {0.0f, 0.0f};
-            if (tid < C) {
-                const float2 p = CLUSTER ? ld_cluster_f2(&s.part[slot], (unsigned)tid) : s.part[slot];
-                v = df{p.x, p.y};
+        // ---- resolve the group in order (warp 0 of every CTA, the same numbers; lane m = trial m)
+        if (warp == 0) {
+            df S = {0.0f, 0.0f};
+            int lg = -1;
+            float2 th = make_float2(0.0f, 0.0f);
+            if (lane < ng) {
+                for (int r = 0; r < C; r++)
+                    for (int p = 0; p < parts; p++) {
+                        const float2 x = xpart[r * kMolWarps + lane * parts + p];
+                        S = df_add(S, df{x.x, x.y});
+                    }
+                const MolTrial &t = d.trials[cursor + lane];
+                lg = t.g;
+                th = make_float2(t.thr_hi, t.thr_lo);
             }
-            v = warp_sum_df(v);
-            v.hi = __shfl_sync(0xffffffffu, v.hi, 0);
-            v.lo = __shfl_sync(0xffffffffu, v.lo, 0);
-            if (tid == 0) {
-                int dec;
-                if (!isfinite(v.hi)) dec = 2;
-                else dec = df_gt(v, df{tr.thr_hi, tr.thr_lo}) ? 0 : 1;
-                s.flag[0] = dec;
-                s.red[0] = make_float2(v.hi, v.lo);
-                if (dec == 1 && cursor + 1 < n && d.trials[cursor + 1].g == tr.g) s.flag[1] = 1;
+            if (EVAL && rank == 0 && lane == 0) *d.eval_du = (double)S.hi + (double)S.lo;
+            uint32_t accm = 0;
+            int done = EVAL ? 0 : ng, bad = 0;
+            for (int a = 0; a < done; a++) {
+                const float2 c = xcorr[a * kMolAhead + min(lane, kMolAhead - 1)];
+                const int ga = __shfl_sync(0xffffffffu, lg, a);
+                // every lane forms its own flags; lane a's are the ones used
+                const int fl = (isfinite(S.hi) ? 0 : 2) | (df_gt(S, df{th.x, th.y}) ? 0 : 1);
+                const int f = __shfl_sync(0xffffffffu, fl, a);
+                if (__ballot_sync(0xffffffffu, lane < a && ((accm >> lane) & 1u) && lg == ga)) {
+                    done = a;   // its molecule was moved by an accepted trial of this group
+                    break;
+                }
+                if (f & 2) {
+                    bad = 1;
+                    done = a;
+                    break;
+                }
+                if (f & 1) {
+                    accm |= 1u << a;
+                    const df Sc = df_add(S, df{c.x, c.y});
+                    const bool later = lane > a && lane < ng && lg != ga;
+                    S.hi = later ? Sc.hi : S.hi;
+                    S.lo = later ? Sc.lo : S.lo;
+                }
+            }
+            // lane m's S is trial m's dU as decided
+            const bool take = lane < done && ((accm >> lane) & 1u);
+            if (rank == 0 && lane < done) {
+                if (d.log_du) d.log_du[cursor + lane] = make_float2(S.hi, S.lo);
+                if (d.log_acc) d.log_acc[cursor + lane] = take ? 1 : 0;
+            }
+            const df sum = warp_sum_df(take ? S : df{0.0f, 0.0f});
+            usum = df_add(usum, sum);
+            utot = df_add(utot, sum);
+            if (lane == 0) {
+                s.info[0] = done;
+                s.info[1] = (int)accm;
+                s.info[2] = bad;
             }
         }
         __syncthreads();
-        const int dec = s.flag[0];
-        const df du = {s.red[0].x, s.red[0].y};
-        if (EVAL) {
-            if (rank == 0 && tid == 0) *d.eval_du = (double)du.hi + (double)du.lo;
-            break;
-        }
-        if (dec == 2) {
-            err |= kMolErrNonFinite;
-            break;
-        }
-        if (rank == 0 && tid == 0) {
-            if (d.log_du) d.log_du[cursor] = make_float2(du.hi, du.lo);
-            if (d.log_acc) d.log_acc[cursor] = (uint8_t)dec;
-        }
-        if (dec == 1) {
-            nacc++;
-            usum = df_add(usum, du);
-            utot = df_add(utot, du);
-            const int gs = d.gs, g = tr.g;
-            const GroupBuf &B = s.buf[b];
-            if (tid < gs) {
-                const int site = g * gs + tid;
+        if (EVAL) break;
+        const int done = s.info[0];
+        const uint32_t accm = (uint32_t)s.info[1];
+        nacc += __popc(accm);
+        // ---- apply the accepted trials (distinct molecules), one warp each
+        for (int m = warp; m < done; m += kMolWarps) {
+            if (!((accm >> m) & 1u)) continue;
+            const GroupBuf B = mol_group(s, d.gs, m);
+            const int g = d.trials[cursor + m].g, gs = d.gs;
+            if (lane < gs) {
+                const int site = g * gs + lane;
                 int64_t *P = d.rep_pos + ((size_t)rank * d.N + site) * 3;
                 double *MU = d.rep_mu + ((size_t)rank * d.N + site) * 3;
-                for (int a = 0; a < 3; a++) {
-                    P[a] = B.gX[3 * tid + a];
-                    MU[a] = B.gmu[3 * tid + a];
+                for (int x = 0; x < 3; x++) {
+                    P[x] = B.gX[3 * lane + x];
+                    MU[x] = B.gmu[3 * lane + x];
                 }
-                const int4 pn = make_int4(B.gn[tid].x, B.gn[tid].y, B.gn[tid].z, B.go[tid].w & 0xFF);
+                const int4 pn = make_int4(B.gn[lane].x, B.gn[lane].y, B.gn[lane].z, B.go[lane].w & 0xFF);
                 if (site >= j0 && site < j1) {
                     if (SLICE_SMEM) s.spos[site - j0] = pn;
                     else d.pos4[site] = pn;
@@ -676,15 +1076,20 @@ __global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc
                 const int k = d.site_dip[site];
                 if (k >= k0 && k < k1) {
                     s.sdpos[k - k0] = make_int4(pn.x, pn.y, pn.z, (site << 8) | (pn.w & 0xFF));
-                    s.sdip[k - k0] = B.gfn[tid];
+                    s.sdip[k - k0] = B.gfn[lane];
                 }
-            } else if (tid == gs) {
+            } else if (lane == gs) {
                 int64_t *CM = d.rep_cm + ((size_t)rank * d.M + g) * 3;
-                for (int a = 0; a < 3; a++) CM[a] = B.gcm[a];
+                for (int x = 0; x < 3; x++) CM[x] = B.gcm[x];
             }
         }
-        __syncthreads();
+        cursor += done;
+        if (s.info[2]) {
+            err |= kMolErrNonFinite;
+            break;
+        }
     }
+    __syncthreads();
     // write the slices back (each CTA its own range) and the scalars
     if (!EVAL) {
         if (SLICE_SMEM)
@@ -704,7 +1109,7 @@ __global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc
             sc->error |= err;
         }
     }
-    if (CLUSTER) cluster_barrier();   // no CTA leaves while another may read its shared memory
+    if (CLUSTER) cluster_barrier();   // no CTA leaves while another may write its shared memory
 }
 
 // Apply an evaluated explicit trial (fg_mol_commit): new positions, dipoles
@@ -911,23 +1316,39 @@ void mol_mass_center(const int64_t *X, int front, int gs, int64_t out[3]) {
     }
 }
 
-size_t mol_smem_bytes(const fg_molsys *h, int C, bool slice_smem) {
+constexpr size_t kMolSmemMax = 220 * 1024;   // of the 227 KB a CTA may hold
+size_t mol_smem_bytes(const fg_molsys *h, int C, bool slice_smem, int ahead) {
     size_t off[16];
-    fgm::mol_smem_layout((h->N + C - 1) / C, (h->D + C - 1) / C, h->gs, slice_smem, off);
-    return off[6];
+    fgm::mol_smem_layout((h->N + C - 1) / C, (h->D + C - 1) / C, h->gs, slice_smem, ahead, off);
+    return off[7];
+}
+// Trials per group of a launch: kMolAhead where their buffers fit beside the
+// site slice, fewer (at least four) where that keeps the slice in shared
+// memory; slice = false: the slice stays in global memory (one buffer where
+// the dipole slice leaves room for no more).
+int mol_ahead(const fg_molsys *h, int C, bool &slice) {
+    slice = true;
+    for (int a = fgm::kMolAhead; a >= 4; a /= 2)
+        if (mol_smem_bytes(h, C, true, a) <= kMolSmemMax) return a;
+    slice = false;
+    int a = fgm::kMolAhead;
+    while (a > 1 && mol_smem_bytes(h, C, false, a) > kMolSmemMax) a /= 2;
+    return a;
 }
 
 struct MolLaunch {
-    void (*fn)(const fgm::MolDesc *);
+    void (*fn)(const fgm::MolDesc *, int, int64_t);
     size_t smem;
+    int ahead;
     bool cluster;
 };
 
 template <bool EVAL>
 int mol_pick(const fg_molsys *h, MolLaunch &L) {
-    const bool slice = mol_smem_bytes(h, h->C, true) <= 200 * 1024;
+    bool slice;
+    L.ahead = mol_ahead(h, h->C, slice);
     const bool cl = h->C > 1;
-    L.smem = mol_smem_bytes(h, h->C, slice);
+    L.smem = mol_smem_bytes(h, h->C, slice, L.ahead);
     L.cluster = cl;
     if (slice) L.fn = cl ? fgm::mol_sweep_kernel<true, true, EVAL> : fgm::mol_sweep_kernel<true, false, EVAL>;
     else L.fn = cl ? fgm::mol_sweep_kernel<false, true, EVAL> : fgm::mol_sweep_kernel<false, false, EVAL>;
@@ -940,7 +1361,8 @@ int mol_pick(const fg_molsys *h, MolLaunch &L) {
     return FG_OK;
 }
 
-int mol_launch(const fg_molsys *h, const MolLaunch &L, const fgm::MolDesc *descs, int n_systems, cudaStream_t st) {
+int mol_launch(const fg_molsys *h, const MolLaunch &L, const fgm::MolDesc *descs, int n_systems, cudaStream_t st,
+               int64_t quantum = INT64_MAX / 2) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(n_systems * h->C));
     cfg.blockDim = dim3(fgm::kMolThreads);
@@ -955,9 +1377,28 @@ int mol_launch(const fg_molsys *h, const MolLaunch &L, const fgm::MolDesc *descs
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, L.fn, descs);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, L.fn, descs, L.ahead, quantum);
     if (e != cudaSuccess) return fail(FG_ERR_CUDA, "molecule sweep launch: %s", cudaGetErrorString(e));
     return FG_OK;
+}
+
+// Clusters of this launch that the device runs at once (0: unknown).
+int mol_slots(const fg_molsys *h, const MolLaunch &L) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)h->C);
+    cfg.blockDim = dim3(fgm::kMolThreads);
+    cfg.dynamicSmemBytes = L.smem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)h->C;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, (const void *)L.fn, &cfg) == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
 }
 
 // Largest cluster the device runs for this kernel's shared memory (<= 16).
@@ -1146,54 +1587,81 @@ int mol_upload(fg_molsys *h, int64_t n, const int32_t *mol, const double *axis, 
 int mol_run(fg_molsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *total) {
     if (!sys || n < 1) return fail(FG_ERR_INVALID, "bad argument");
     fg_molsys *h0 = sys[0];
-    size_t smem_slice = 0, smem_flat = 0;
     bool all_slice = true;
+    int ahead = fgm::kMolAhead;   // group buffers that fit every system
     int64_t maxn = 0;
     for (int i = 0; i < n; i++) {
         fg_molsys *h = sys[i];
         if (!h || !h->state_set) return fail(FG_ERR_STATE, "system %d has no state", i);
         if (h->C != h0->C) return fail(FG_ERR_INVALID, "systems must share the cluster size");
         if (h->device != h0->device) return fail(FG_ERR_INVALID, "systems must share the device");
-        const size_t a = mol_smem_bytes(h, h->C, true);
-        if (a > 200 * 1024) all_slice = false;
-        smem_slice = std::max(smem_slice, a);
-        smem_flat = std::max(smem_flat, mol_smem_bytes(h, h->C, false));
+        bool slice;
+        const int a = mol_ahead(h, h->C, slice);
+        if (!slice) all_slice = false;
+        ahead = std::min(ahead, a);
         maxn = std::max(maxn, h->n_stream);
         CK(cudaStreamSynchronize(h->stream));
     }
     MolLaunch L;
     L.cluster = h0->C > 1;
-    L.smem = all_slice ? smem_slice : smem_flat;
+    L.ahead = ahead;
+    L.smem = 0;
+    for (int i = 0; i < n; i++) L.smem = std::max(L.smem, mol_smem_bytes(sys[i], sys[i]->C, all_slice, ahead));
     if (all_slice) L.fn = L.cluster ? fgm::mol_sweep_kernel<true, true, false> : fgm::mol_sweep_kernel<true, false, false>;
     else L.fn = L.cluster ? fgm::mol_sweep_kernel<false, true, false> : fgm::mol_sweep_kernel<false, false, false>;
     CK(cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
     if (L.cluster) CK(cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    // A last wave of clusters that is nearly empty costs as much as a full one
+    // (at C = 4 the GPU holds 36 clusters at once: 38 systems ran 2 waves for
+    // 1.06 waves' work). Where more than a tenth would be lost, the systems
+    // take turns: launches of exactly `slots` clusters run `quantum` trials of
+    // each, in rotation, so that all of them are full.
+    const int64_t kChunk = 65536;   // most trials of one launch
+    int slots = n;
+    int64_t quantum = kChunk;
+    const int fit = mol_slots(h0, L);
+    if (fit > 0 && fit < n) {
+        const int waves = (n + fit - 1) / fit;
+        if (10 * n < 9 * waves * fit) {
+            double best = waves;
+            for (int q = 2; q <= 16; q++) {   // turns per system; whole groups each
+                const int64_t qu = ((maxn + q - 1) / q + fgm::kMolAhead - 1) / fgm::kMolAhead * fgm::kMolAhead;
+                const int64_t turns = (maxn + qu - 1) / qu, rounds = (turns * n + fit - 1) / fit;
+                // in waves of maxn trials; a launch lasts as long as its unluckiest system, whose
+                // groups ended early on a molecule met twice (about 6 trials at 1000 molecules)
+                const double cost = (double)rounds * (qu + 6) / maxn;
+                if (qu <= kChunk && cost < best) {
+                    best = cost;
+                    slots = fit;
+                    quantum = qu;
+                }
+            }
+        }
+    }
     cudaStream_t st = h0->stream;
     const fgm::MolDesc *descs = h0->d_desc;
     fgm::MolDesc *tmp = nullptr;
-    if (n > 1) {
-        std::vector<fgm::MolDesc> v(n);
-        for (int i = 0; i < n; i++) v[i] = sys[i]->desc;
-        CK(cudaMalloc(&tmp, n * sizeof(fgm::MolDesc)));
-        CK(cudaMemcpyAsync(tmp, v.data(), n * sizeof(fgm::MolDesc), cudaMemcpyHostToDevice, st));
+    if (n > 1) {   // twice in a row, so that any rotation is one piece
+        std::vector<fgm::MolDesc> v(2 * (size_t)n);
+        for (int i = 0; i < n; i++) v[i] = v[n + i] = sys[i]->desc;
+        CK(cudaMalloc(&tmp, v.size() * sizeof(fgm::MolDesc)));
+        CK(cudaMemcpyAsync(tmp, v.data(), v.size() * sizeof(fgm::MolDesc), cudaMemcpyHostToDevice, st));
         descs = tmp;
     }
     std::vector<fgm::MolScalars> s0(n), s1(n);
     for (int i = 0; i < n; i++) {
         CK(cudaMemcpyAsync(&s0[i], sys[i]->sc, sizeof(fgm::MolScalars), cudaMemcpyDeviceToHost, st));
     }
-    const int64_t kChunk = 65536;
-    const int64_t nl = (maxn + kChunk - 1) / kChunk;
-    std::vector<int64_t> ends((size_t)nl * n);
     CK(cudaEventRecord(h0->ev0, st));
     int rc = FG_OK;
-    for (int64_t c = 0; c < nl && !rc; c++) {
-        for (int i = 0; i < n; i++) {
-            int64_t &e = ends[(size_t)c * n + i];
-            e = std::min(sys[i]->n_stream, (c + 1) * kChunk);
-            CK(cudaMemcpyAsync(&sys[i]->sc->n_trials, &e, sizeof(int64_t), cudaMemcpyHostToDevice, st));
-        }
-        rc = mol_launch(h0, L, descs, n, st);
+    int64_t nl = 0;
+    if (slots >= n) {
+        for (int64_t c = 0; c < maxn && !rc; c += kChunk, nl++) rc = mol_launch(h0, L, descs, n, st, kChunk);
+    } else {
+        // round r runs the systems (r slots + i) mod n, i < slots, for one quantum each
+        const int64_t rounds = ((maxn + quantum - 1) / quantum * n + slots - 1) / slots;
+        for (int64_t r = 0; r < rounds && !rc; r++, nl++)
+            rc = mol_launch(h0, L, descs + r * slots % n, slots, st, quantum);
     }
     CK(cudaEventRecord(h0->ev1, st));
     CK(cudaEventSynchronize(h0->ev1));

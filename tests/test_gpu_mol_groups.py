@@ -1,0 +1,75 @@
+"""Groups of trials in the molecule sweep: the shapes where the grouped path can
+go wrong (molecules met twice in a group, one site per molecule, the largest
+molecule, molecules longer than the cutoff, dipoles on every site, non-uniform
+LJ tables, boxes with unequal sides), and systems that take turns because
+their clusters do not all fit the GPU."""
+import numpy as np
+import pytest
+
+from beofaunus_gb300 import workloads
+from beofaunus_gb300.gpu import MolSystem, mol_draw_stream, mol_run_many
+from oracle.oracle import OracleMol
+
+pytestmark = pytest.mark.gpu
+
+
+def molecules(case):
+    kw = dict(n_mol=case["m"], seed=70 + case["m"], molsize=case["gs"], box=case.get("box"), cutoff=case.get("rc", 12.0))
+    if "radius" in case:
+        kw["mol_radius"] = case["radius"]
+    p, x, mu, mus, ids = workloads.dipolar_molecules(**kw)
+    if case.get("tables"):
+        for t, (s, e) in enumerate(((3.5, 0.2), (3.0, 0.35), (4.0, 0.1))):
+            p.type_sigma[t], p.type_eps[t] = s, e
+    if case.get("skew"):   # the same coordinates in a longer, unequal box
+        p.box[1] *= 1.07
+        p.box[2] *= 1.21
+    if case.get("dipoles"):
+        rng = np.random.default_rng(5)
+        mu = rng.normal(size=x.shape)
+        mu /= np.linalg.norm(mu, axis=1, keepdims=True)
+        mus = np.where(np.arange(len(mus)) % 3 < 2, 0.3, 0.0)
+    return p, x, mu, mus, ids
+
+
+CASES = [dict(m=3, gs=20, box=50.0), dict(m=17, gs=1, box=48.0), dict(m=40, gs=31, box=70.0), dict(m=33, gs=5, box=45.0, tables=True),
+         dict(m=33, gs=6, box=45.0, skew=True), dict(m=20, gs=7, box=45.0, dipoles=True), dict(m=9, gs=4, box=80.0, rc=6.0, radius=14.0),
+         dict(m=130, gs=9, box=75.0, tables=True, skew=True, dipoles=True)]
+
+
+@pytest.mark.parametrize("cluster", [1, 4])
+@pytest.mark.parametrize("case", CASES, ids=[str(i) for i in range(len(CASES))])
+def test_grouped_sweep_matches_oracle(case, cluster):
+    """FP32 pair terms: a few roundings (6e-8) of each near term and of the
+    larger dU of a close contact: 1e-6 kT + 4e-7 |dU|."""
+    p, x, mu, mus, ids = molecules(case)
+    s = MolSystem(p, x, mu, mus, ids, case["gs"], cluster=cluster)
+    o = OracleMol(p, x, mu, mus, ids, case["gs"])
+    st = mol_draw_stream(12, case["m"], 150, 1.0, 0.3, True)
+    r, ro = s.sweep(st), o.run_stream(st)
+    np.testing.assert_array_equal(r["acc"], ro["acc"])
+    assert np.all(np.abs(r["du"] - ro["du"]) < 1e-6 + 4e-7 * np.abs(ro["du"]))
+    xyz, mu1, _ = s.state()
+    xo, mo = o.state()[:2]
+    L = np.array(p.box[:3])
+    d = xyz - xo
+    assert np.abs(d - L * np.round(d / L)).max() < 1e-9
+    assert np.abs(mu1 - mo).max() < 1e-12
+
+
+def test_systems_in_turns_equal_alone():
+    """More clusters than the GPU holds at once, uneven streams: every system
+    ends exactly where it ends alone."""
+    data = [workloads.dipolar_molecules(20 + k % 3, seed=k, molsize=6) for k in range(41)]
+    streams = [mol_draw_stream(900 + k, 20 + k % 3, 40 + 7 * (k % 5), 1.0, 0.3, True) for k in range(41)]
+    many = [MolSystem(p, x, mu, mus, ids, 6, cluster=4) for (p, x, mu, mus, ids) in data]
+    for s, st in zip(many, streams):
+        s.stream_upload(st)
+    per, _ = mol_run_many(many)
+    for k in (0, 7, 35, 36, 40):
+        p, x, mu, mus, ids = data[k]
+        alone = MolSystem(p, x, mu, mus, ids, 6, cluster=4)
+        r = alone.sweep(streams[k])
+        assert per[k]["trials"] == len(streams[k]["u"]) and per[k]["accepted"] == r["acc"].sum()
+        for a, b in zip(many[k].state(), alone.state()):
+            np.testing.assert_array_equal(a, b)
