@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <mutex>
 #include <random>
@@ -475,10 +476,10 @@ bool dh_block_ok(const fg_system *h) { return h->model == FG_MODEL_DH_LJ && !h->
 // CTA's particles are staged in shared memory.
 size_t dh_block_smem(int N, int C, bool *slice) {
     const int ns = (N + C - 1) / C;
-    const size_t with = fg::blk_smem_bytes(ns, true);
+    const size_t with = fg::blk_smem_bytes(ns, true, C);
     const bool fits = with + sizeof(SysDesc) + 1024 <= 227 * 1024;
     if (slice) *slice = fits;
-    return fits ? with : fg::blk_smem_bytes(ns, false);
+    return fits ? with : fg::blk_smem_bytes(ns, false, C);
 }
 
 BlkFn dh_block_fn(bool slice, bool cluster) {
@@ -535,6 +536,7 @@ int dh_block_max_cluster() {
 std::mutex g_tune_mu;
 std::map<int, int> g_tune_dh_ctas;   // floor(log2 N) -> CTAs
 int g_tune_min_per_cta = 256;
+bool g_tune_min_set = false;          // chosen by fg_batch_autotune
 int g_tune_dip_threads = 0;          // threads per point-dipole system (0: built-in default)
 
 int size_class(int N) {
@@ -543,8 +545,12 @@ int size_class(int N) {
     return c;
 }
 
-// CTAs for one system alone: the tuned choice for its size class, else about
-// 2048 particles per CTA.
+// CTAs for one system alone: the tuned choice for its size class, else as many
+// as keep at least 64 particles each. A block of 32 trials costs about 0.33 us
+// per trial on any number of CTAs and 0.4 ns per particle of a CTA's slice, so
+// more CTAs always help down to slices of 64 (us per trial, 1 / 4 / 16 CTAs:
+// 256 particles 0.67 / 0.49 / -, 2001 1.29 / 0.54 / 0.38, 16384 8.9 / 2.0 / 0.72).
+constexpr int kDhMinPerCta = 64;
 int dh_block_ctas(int N) {
     const int maxc = dh_block_max_cluster();
     {
@@ -553,12 +559,19 @@ int dh_block_ctas(int N) {
         if (it != g_tune_dh_ctas.end()) return std::max(1, std::min(it->second, maxc));
     }
     int C = 1;
-    while (C < maxc && (N + C - 1) / C > 2048) C <<= 1;
+    while (2 * C <= maxc && N / (2 * C) >= kDhMinPerCta) C <<= 1;
     return C;
 }
 int tuned_min_per_cta() {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     return g_tune_min_per_cta;
+}
+// Batches and tempering: the tuned choice, else slices down to kDhMinPerCta (the
+// job server keeps tuned_min_per_cta's default, which also sizes its rounds
+// and so its memory budget).
+int batch_min_per_cta() {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    return g_tune_min_set ? g_tune_min_per_cta : kDhMinPerCta;
 }
 
 int dh_sm_count() {
@@ -568,28 +581,81 @@ int dh_sm_count() {
     return std::max(n, 1);
 }
 
+// Clusters of c CTAs of the block kernel that the device runs at once, c = 1,
+// 2, 4, 8, 16 (index log2 c): fewer SMs than there are, since a cluster stays
+// within a GPC (152, 76, 36, 15 and 7 on 152 SMs).
+const int *dh_cluster_slots() {
+    static int cached[64][5];
+    static bool init[64] = {};
+    static std::mutex mu;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    dev = std::min(std::max(dev, 0), 63);
+    std::lock_guard<std::mutex> lk(mu);
+    if (init[dev]) return cached[dev];
+    for (int k = 0; k < 5; k++) {
+        const int c = 1 << k;
+        cached[dev][k] = dh_sm_count() / c;
+        if (c == 1 || c > dh_block_max_cluster()) continue;
+        bool slice;
+        const size_t smem = dh_block_smem(1024 * c, c, &slice);
+        BlkFn fn = dh_block_fn(slice, true);
+        if (dh_block_attrs(fn, smem, true)) continue;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)c);
+        cfg.blockDim = dim3(fg::kBlkThreads);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)c;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, (const void *)fn, &cfg) == cudaSuccess && n > 0) cached[dev][k] = n;
+        else cudaGetLastError();
+    }
+    init[dev] = true;
+    return cached[dev];
+}
+
 // CTAs per system for systems run side by side: start at one each, then keep
-// doubling the system with the most work per CTA (weight / CTAs) while the
-// SMs hold every CTA at once, the device allows the cluster and each CTA keeps
-// at least min_per_cta particles. weight ~ pair evaluations of the launch.
+// doubling the system that would take longest (weight w ~ pair evaluations of
+// the launch, so w / N trials of about 0.35 us plus 0.4 ns per particle of a
+// slice each) while every cluster still runs at once, the device allows the
+// cluster and each CTA keeps at least min_per_cta particles. At once: for each
+// size c the clusters of at least c CTAs, cut into pieces of c, must fit the
+// device's slots for c (a cluster that had to wait would add its whole time).
 std::vector<int> dh_block_ctas_many(const std::vector<int> &N, const std::vector<double> &w, int min_per_cta) {
     const int n = (int)N.size();
     std::vector<int> C(n, 1);
     const int maxc = dh_block_max_cluster();
-    long spare = (long)dh_sm_count() - n;
-    while (spare > 0) {
+    const int *slots = dh_cluster_slots();
+    long used[5] = {n, 0, 0, 0, 0};   // pieces of 1 << k CTAs
+    std::vector<char> full(n, 0);
+    while (true) {
         int best = -1;
         double bw = 0;
         for (int i = 0; i < n; i++) {
-            if (2 * C[i] > maxc || N[i] / (2 * C[i]) < min_per_cta || C[i] > spare) continue;
-            const double x = w[i] / C[i];
+            if (full[i] || 2 * C[i] > maxc || N[i] / (2 * C[i]) < min_per_cta) continue;
+            const double x = w[i] / N[i] * (850.0 + (double)N[i] / C[i]);
             if (x > bw) {
                 bw = x;
                 best = i;
             }
         }
         if (best < 0) break;
-        spare -= C[best];
+        // doubling adds C / c pieces at every size c <= C and one piece of 2 C
+        const int c = C[best];
+        bool ok = true;
+        for (int k = 0; k < 5 && (1 << k) <= 2 * c; k++)
+            if (used[k] + ((1 << k) <= c ? c >> k : 1) > slots[k]) ok = false;
+        if (!ok) {
+            full[best] = 1;
+            continue;
+        }
+        for (int k = 0; k < 5 && (1 << k) <= 2 * c; k++) used[k] += (1 << k) <= c ? c >> k : 1;
         C[best] *= 2;
     }
     return C;
@@ -667,16 +733,21 @@ int dh_groups_build_c(DhGroups &g, const std::vector<int> &N, const std::vector<
     g.mem.clear();
     g.maxN.clear();
     g.offset.clear();
-    for (size_t i = 0; i < N.size(); i++) {
-        size_t k = 0;
-        while (k < g.C.size() && g.C[k] != C[i]) k++;
-        if (k == g.C.size()) {
-            g.C.push_back(C[i]);
-            g.mem.emplace_back();
-            g.maxN.push_back(0);
+    // the largest clusters first: they need that many free SMs within one GPC,
+    // which the small ones, placed first, would scatter over (64 replicas: the
+    // two 16-CTA systems started after the others' 4.7 ms)
+    std::vector<int> sizes(C.begin(), C.end());
+    std::sort(sizes.begin(), sizes.end(), std::greater<int>());
+    sizes.erase(std::unique(sizes.begin(), sizes.end()), sizes.end());
+    for (int c : sizes) {
+        g.C.push_back(c);
+        g.mem.emplace_back();
+        g.maxN.push_back(0);
+        for (size_t i = 0; i < N.size(); i++) {
+            if (C[i] != c) continue;
+            g.mem.back().push_back((int)i);
+            g.maxN.back() = std::max(g.maxN.back(), N[i]);
         }
-        g.mem[k].push_back((int)i);
-        g.maxN[k] = std::max(g.maxN[k], N[i]);
     }
     std::vector<int> all;
     for (auto &m : g.mem) {

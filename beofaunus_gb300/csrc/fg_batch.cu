@@ -175,7 +175,7 @@ int batch_config(fg_batch *b) {
         w.push_back((double)h->N * h->N);   // a sweep of N trials over N partners
     }
     if (b->dh_block)   // the one-CTA kernel (cfg.fn) is not launched for these members
-        return dh_groups_build(b->dh, Ns, w, b->min_per_cta > 0 ? b->min_per_cta : tuned_min_per_cta());
+        return dh_groups_build(b->dh, Ns, w, b->min_per_cta > 0 ? b->min_per_cta : batch_min_per_cta());
     return set_smem_attr((const void *)b->cfg.fn, sm);
 }
 

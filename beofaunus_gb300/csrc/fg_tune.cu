@@ -162,6 +162,7 @@ int fg_batch_autotune(fg_batch *b, int64_t n_trials, fg_tune_report *report) {
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tune_min_per_cta = t[best].first;
+        g_tune_min_set = true;
     }
     if (b->graph) {   // a captured round holds the old launch shapes
         cudaGraphExecDestroy(b->graph);
@@ -217,6 +218,7 @@ int fg_tune_reset(void) {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune_dh_ctas.clear();
     g_tune_min_per_cta = 256;
+    g_tune_min_set = false;
     g_tune_dip_threads = 0;
     return FG_OK;
 }
