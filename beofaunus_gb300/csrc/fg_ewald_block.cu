@@ -10,7 +10,10 @@
 //   real space   [u(n_m,n_a) - u(o_m,n_a)] - [u(n_m,o_a) - u(o_m,o_a)]
 //   surface      2 c dM_a . dM_m                 (E_surf = c |M|^2)
 //   reciprocal   sum_k A'_k 2 Re(conj(D_a,k) D_m,k)
-// with D_m,k = q e^{ik.r_old}(e^{ik.d} - 1) the same increment the energy uses.
+// with D_m,k = q (e^{ik.r_new} - e^{ik.r_old}) = 2 q sin(k.d / 2) i e^{ik.r_mid},
+// r_mid the step's midpoint, the same increment the energy uses (its error is
+// relative to |d|, and a real sine times a phase takes 10 of the 65 slots that
+// q e^{ik.r_old}(e^{ik.d} - 1) took less).
 // The reciprocal parts of all pairs of the block form a 32 x 32 Gram matrix
 // over k of the trials' increments; it is accumulated in 4 x 4 register tiles
 // while the increments stream through shared memory in chunks of k-vectors.
@@ -122,11 +125,12 @@ __device__ inline EbSmem eb_carve(char *base, const SysDesc &d, bool cells) {
 // the two 16-row tiles and, G being X X^T, the B fragments of the four
 // 8-column tiles. Accumulated tiles (row tile, column tile): (0,0) (0,1)
 // (0,2) (0,3) (1,2) (1,3), every pair a < m lies in one of them.
-__device__ __forceinline__ uint32_t eb_tf32(float x) {
-    uint32_t r;
-    asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
-    return r;
-}
+// x rounded to TF32 (to nearest, ties away: the bits of cvt.rna.tf32.f32 for
+// finite x) with integer instructions: the conversion runs on the SFU, and 16
+// of them per k-step and warp were 128 of the step's 480 cycles. (A NaN may
+// lose itself here; the trial's reciprocal base, FP32 sums of the same
+// amplitudes, keeps it.)
+__device__ __forceinline__ uint32_t eb_tf32(float x) { return (__float_as_uint(x) + 0x1000u) & 0xFFFFE000u; }
 __device__ __forceinline__ void eb_mma(float c[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                  "{%0,%1,%2,%3};"
@@ -153,6 +157,15 @@ __device__ __forceinline__ void eb_gram_regs(const float xf[4][2], float gc[6][4
     }
 }
 
+// sin(x) with error relative to x for |x| <= 0.8 (next term < 3e-9 of it).
+__device__ __forceinline__ float eb_sin(float x) {
+    const float x2 = x * x;
+    float s = fmaf(x2, 2.7557319223985893e-06f, -1.9841269841269841e-04f);
+    s = fmaf(x2, s, 8.3333333333333333e-03f);
+    s = fmaf(x2, s, -1.6666666666666667e-01f);
+    return fmaf(x2 * x, s, x);
+}
+
 // Barrier 1 over the block's warps 1.. (nthreads = blockDim - 32 threads).
 __device__ __forceinline__ void eb_qbar(int nthreads) {
     asm volatile("bar.sync 1, %0;" ::"r"(nthreads) : "memory");
@@ -177,79 +190,268 @@ __device__ __forceinline__ void eb_st_remote(int *p, unsigned rank, int v) {
 }
 
 // Real-space base of one trial by one warp (or part `part` of `nparts`: the
-// candidate batches part, part + nparts, ...). Candidates (cell stencil, or all
-// particles) are screened by distance first: only those that may lie within
-// reach2 of the old or the new position (all particles: either distance; cell
-// stencil: the distance to the step's midpoint against reach + |d|/2) enter a
-// 32-entry warp queue in shared memory (qp, qm), which is evaluated with all
-// lanes busy when the next batch would overflow it. Skipped candidates
-// contribute exactly zero (every pair term is zero beyond reach2), so the sum
-// is that of the full loop, in another order.
+// candidate batches part, part + nparts, ...). The phase is bound by issue
+// slots, so each stage does as little as it can for as many as it must see:
+// 1. Batches of 32 slots (of a stencil cell, or of all particles) are screened
+//    by the distance to the step's midpoint against reach + |d|/2; all that is
+//    kept of a batch is the ballot, in lane (batch mod 32). Skipped candidates
+//    contribute exactly zero (every pair term is zero beyond reach2).
+// 2. Every 32 batches the lanes write the slots of their set bits to a list.
+// 3. The list is evaluated 32 at a time with all lanes busy.
+// 4. Those within 1.5 sigma of either position (four a trial at 0.0037 ions per
+//    cubic Angstrom) need erfcf, a correctly rounded root and divide or the
+//    double-float core, some 2 k issue slots against 0.2 k: they wait in a
+//    queue until both of the warp's trials are walked and are evaluated
+//    together, two lanes per candidate (new and old position).
+// One block of 32 trials on one CTA, cycles: 49 k -> 32 k at 800 ions without
+// cells, 86 k -> 54 k at 16384 ions with cells, against queueing every screened
+// pair with its position and a near pair in the batch where it was met.
+constexpr int kEbNear = 16;      // entries of the near queue
+constexpr int kEbList = 160;     // entries of the list
+constexpr int kEbBatch = 64;     // cell batches listed at a time
+constexpr int kEbQueueBytes = kEbNear * 24 + kEbList * 4 + kEbBatch * 8;   // of one warp
+// s.delta before the sums are formed: the warps' queues, the trial records
+// (2 x 16 bytes each), and from 28 KB the reciprocal-base partials
+constexpr int kEbRecords = (kEbThreads / 32) * kEbQueueBytes;
+static_assert(kEbRecords + 32 * kEbTrials <= 28672 && 28672 + 8 * kEbThreads <= 8 * kEbKc * kEbTrials, "eb scratch");
+struct EbQueue {
+    int4 *np;        // near queue: positions
+    int2 *nm, *bat;  // near queue: slot, type + 256 x which of the warp's trials; batches: first slot, count
+    int *list;       // slots within reach
+    int nn;          // near queue length
+};
+__device__ __forceinline__ EbQueue eb_queue(void *base) {
+    EbQueue q;
+    q.np = reinterpret_cast<int4 *>(base);
+    q.nm = reinterpret_cast<int2 *>(q.np + kEbNear);
+    q.bat = q.nm + kEbNear;
+    q.list = reinterpret_cast<int *>(q.bat + kEbBatch);
+    q.nn = 0;
+    return q;
+}
+// What a far pair needs of its trial, in registers.
+struct EbFar {
+    int ho[3], hn[3], hm[3];   // old, new position and their midpoint
+    float q, qe;               // charge; qeqe of the single type
+    float near2, rm2;          // squared distances: near pair, reach from the midpoint
+    float sl[3];               // the axis factors (the descriptor lies in shared memory
+                               // and would be read again after each warp barrier)
+};
+__device__ __forceinline__ float eb_r2(int4 a, const int h[3], const EbFar &m) {
+    const float x = (float)(a.x - h[0]) * m.sl[0], y = (float)(a.y - h[1]) * m.sl[1], z = (float)(a.z - h[2]) * m.sl[2];
+    return fmaf(x, x, fmaf(y, y, z * z));
+}
+// rsqrt_nr and erfc_nr for arguments that are neither subnormal nor huge:
+// without the range checks of rsqrtf and __frcp_rn (a reciprocal after one
+// Newton step).
+__device__ __forceinline__ float eb_rsqrt(float r2) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(r2));
+    return y * fmaf(-0.5f * r2 * y, y, 1.5f);
+}
+__device__ __forceinline__ float eb_erfc(float z) {
+    const float x = fmaf(0.5f, z, 1.0f);
+    float t;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(x));
+    t = fmaf(t, fmaf(-x, t, 1.0f), t);
+    return erfc_nr_at(t, z);
+}
+// u(new) - u(old) of a pair beyond 1.5 sigma of both positions: no WCA, no
+// core; pair_ewald_wca<false>'s real-space term at both, without branches.
+__device__ __forceinline__ float eb_far(const EbFar &m, float r2n, float r2o, float qj, int t, const SysDesc &d) {
+    const float qq = m.q * qj * (d.uniform_types ? m.qe : d.qeqe[t]) * d.lB;
+    float un, uo;
+    if (d.kappa == 0.0f) {
+        const float in = eb_rsqrt(r2n), io = eb_rsqrt(r2o);
+        const float en = eb_erfc(d.alpha * (r2n * in)), eo = eb_erfc(d.alpha * (r2o * io));
+        un = r2n <= d.rc2 ? qq * en * in : 0.0f;
+        uo = r2o <= d.rc2 ? qq * eo * io : 0.0f;
+    } else {
+        un = pair_ewald_wca<false>(r2n, qq, 0.0f, 0.0f, 0.0f, d);
+        uo = pair_ewald_wca<false>(r2o, qq, 0.0f, 0.0f, 0.0f, d);
+    }
+    return un - uo;
+}
+// The near queue's sum: lanes 2 e and 2 e + 1 take candidate e at the new and at
+// the old position (with the opposite sign); which: the trial it belongs to.
+__device__ __noinline__ df eb_near(const int4 *np, const int2 *nm, int n, const Move *m0, const Move *m1,
+                                   const short4 *ext, const SysDesc &d, int &which) {
+    const int lane = threadIdx.x & 31, e = lane >> 1;
+    which = 0;
+    if (e >= n) return df{0.0f, 0.0f};
+    const int4 p = np[e];
+    const int2 r = nm[e];
+    which = r.y >> 8;
+    const Move &m = which ? *m1 : *m0;
+    const bool old = lane & 1;
+    const int h0 = old ? m.ho[0] : m.hn[0], h1 = old ? m.ho[1] : m.hn[1], h2 = old ? m.ho[2] : m.hn[2];
+    const float qj = __int_as_float(p.w), r2 = dist2(p, h0, h1, h2, d);
+    const int t = d.uniform_types ? 0 : m.ti * d.n_types + (r.y & 255);
+    df u;
+    if (d.core_tab_n > 0 && r2 < d.s2[t]) {
+        const short4 x = ext[r.x];
+        u = pair_core_df<MODEL_EWALD>(p.x - h0, p.y - h1, p.z - h2, x.x - (old ? m.eo[0] : m.en[0]),
+                                      x.y - (old ? m.eo[1] : m.en[1]), x.z - (old ? m.eo[2] : m.en[2]), m.q, qj, t, d);
+    } else {
+        u = df{pair_u<MODEL_EWALD, true>(r2, m.q, qj, t, d), 0.0f};
+    }
+    return old ? df_neg(u) : u;
+}
+// A warp's sums of its two trials; EbWalk::near empties the near queue into them.
+struct EbWalk {
+    const Move *m[2];
+    float f;       // far pairs of the trial being walked
+    df a0, a1;     // near pairs of either trial
+};
 template <bool CELLS>
-__device__ __forceinline__ void eb_flush(int qn, const int4 *qp, const int2 *qm, const Move &m, const SysDesc &d,
-                                         float &accf, df &accd) {
-    const int lane = threadIdx.x & 31;
+__device__ __forceinline__ void eb_flush_near(EbQueue &q, EbWalk &w, const SysDesc &d) {
+    if (!q.nn) return;   // warp-uniform
     __syncwarp();
-    if (lane < qn) {
-        const int2 e = qm[lane];
-        pair_candidate<MODEL_EWALD>(m, qp[lane], e.y, (CELLS ? d.cell_ext : d.pos_ext) + e.x, d, accf, accd);
+    int which;
+    const df v = eb_near(q.np, q.nm, q.nn, w.m[0], w.m[1], CELLS ? d.cell_ext : d.pos_ext, d, which);
+    if (which) w.a1 = df_add(w.a1, v);
+    else w.a0 = df_add(w.a0, v);
+    __syncwarp();
+    q.nn = 0;
+}
+// Evaluates n listed slots: far pairs at once, near ones into their queue.
+template <bool CELLS>
+__device__ __forceinline__ void eb_eval(int n, EbQueue &q, const EbFar &fm, int which, EbWalk &w, const SysDesc &d) {
+    const int lane = threadIdx.x & 31;
+    const Move &m = *w.m[which];
+    __syncwarp();
+    for (int e = 0; e < n; e += 32) {
+        const bool in = e + lane < n;
+        int idx = 0, t = 0;
+        int4 p = make_int4(0, 0, 0, 0);
+        bool nr = false;
+        if (in) {
+            idx = q.list[e + lane];
+            p = (CELLS ? d.cell_pos : d.pos4)[idx];
+            if (!d.uniform_types) t = CELLS ? d.cell_pid[idx] >> 24 : d.ptype[idx];
+            const float r2n = eb_r2(p, fm.hn, fm), r2o = eb_r2(p, fm.ho, fm);
+            nr = fminf(r2n, r2o) <= fm.near2;
+            if (!nr) w.f += eb_far(fm, r2n, r2o, __int_as_float(p.w), m.ti * d.n_types + t, d);
+            else nr = (CELLS ? d.cell_pid[idx] & 0xFFFFFF : idx) != m.i;   // itself is as near as can be
+        }
+        uint32_t nmask = __ballot_sync(0xffffffffu, nr);
+        while (nmask) {   // warp-uniform
+            if (q.nn == kEbNear) eb_flush_near<CELLS>(q, w, d);
+            const int r = q.nn + __popc(nmask & ((1u << lane) - 1u));
+            if (nr && r < kEbNear) {
+                q.np[r] = p;
+                q.nm[r] = make_int2(idx, t | which << 8);
+                nr = false;
+            }
+            q.nn = min(q.nn + __popc(nmask), kEbNear);
+            nmask = __ballot_sync(0xffffffffu, nr);
+        }
     }
     __syncwarp();
 }
+// Up to 32 batches: batch b takes the slots from base + b step (N in all), or
+// those of the cell batch q.bat[base + b].
 template <bool CELLS>
-__device__ __forceinline__ void eb_push(bool f, int4 pos, int idx, int t, int &qn, int4 *qp, int2 *qm,
-                                        const Move &m, const SysDesc &d, float &accf, df &accd) {
-    const int lane = threadIdx.x & 31;
-    const uint32_t mask = __ballot_sync(0xffffffffu, f);
-    const int c = __popc(mask);
-    if (qn + c > 32) {
-        eb_flush<CELLS>(qn, qp, qm, m, d, accf, accd);
-        qn = 0;
+__device__ __forceinline__ void eb_screen(int base, int step, int nb, EbQueue &q, const EbFar &fm, int which, EbWalk &w,
+                                          const SysDesc &d) {
+    constexpr int U = 4;   // batches a turn; the next turn's records are loaded meanwhile
+    const int lane = threadIdx.x & 31, N = d.N;
+    const int4 *const pos = (CELLS ? d.cell_pos : d.pos4) + lane;
+    uint32_t mask = 0;
+    int4 p[U];
+    bool in[U];
+    auto load = [&](int b) {
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            in[u] = false;
+            if (b + u >= nb) continue;   // warp-uniform
+            const int2 e = CELLS ? q.bat[base + b + u] : make_int2(base + (b + u) * step, N - (base + (b + u) * step));
+            in[u] = lane < e.y;
+            if (in[u]) p[u] = pos[e.x];
+        }
+    };
+#pragma unroll
+    for (int u = 0; u < U; u++) p[u] = make_int4(0, 0, 0, 0);
+    load(0);
+    for (int b = 0; b < nb; b += U) {   // warp-uniform
+        bool f[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) f[u] = in[u] && eb_r2(p[u], fm.hm, fm) <= fm.rm2;
+        load(b + U);
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t v = __ballot_sync(0xffffffffu, f[u]);
+            if (lane == b + u) mask = v;
+        }
     }
-    if (f) {
-        const int r = qn + __popc(mask & ((1u << lane) - 1u));
-        qp[r] = pos;
-        qm[r] = make_int2(idx, t);
+    const int first = lane >= nb ? 0 : CELLS ? q.bat[base + lane].x : base + lane * step;
+    int inc = __popc(mask);
+    const int own = inc;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += v;
     }
-    qn += c;
-}
-__device__ __forceinline__ bool eb_in_reach(int4 p, const Move &m, const SysDesc &d) {
-    return dist2(p, m.hn[0], m.hn[1], m.hn[2], d) <= d.reach2 || dist2(p, m.ho[0], m.ho[1], m.ho[2], d) <= d.reach2;
+    const int total = __shfl_sync(0xffffffffu, inc, 31);
+    int r = inc - own;
+    for (int w0 = 0; w0 < total; w0 += kEbList) {   // warp-uniform
+        while (mask && r < w0 + kEbList) {
+            const int bit = 31 - __clz(mask);
+            mask ^= 1u << bit;
+            q.list[r - w0] = first + bit;
+            r++;
+        }
+        eb_eval<CELLS>(min(total - w0, kEbList), q, fm, which, w, d);
+    }
 }
 
 template <bool CELLS>
-__device__ __forceinline__ void eb_pairs_warp(const Move &m, const SysDesc &d, const Smem &s, int4 *qp, int2 *qm,
-                                              int part, int nparts, float &accf, df &accd) {
+__device__ __forceinline__ void eb_pairs_warp(int which, EbWalk &w, const SysDesc &d, const Smem &s, EbQueue &q,
+                                              float near2, int part, int nparts) {
+    const Move &m = *w.m[which];
     const int lane = threadIdx.x & 31;
-    int qn = 0;
+    // a partner within reach of the old or the new position lies within
+    // reach + |d|/2 of the midpoint (a small margin covers the float rounding)
+    const float reach2m = d.reach2 * 1.0001f + 1e-3f;
+    const float hd = 0.5f * sqrtf(fmaf(m.dxf[0], m.dxf[0], fmaf(m.dxf[1], m.dxf[1], m.dxf[2] * m.dxf[2])));
+    const float rm = sqrtf(reach2m) + hd + 1e-3f;
+    EbFar fm;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        fm.ho[a] = m.ho[a];
+        fm.hn[a] = m.hn[a];
+        fm.hm[a] = m.ho[a] + ((int)(m.hn[a] - m.ho[a]) >> 1);
+        fm.sl[a] = d.s32[a];
+    }
+    fm.q = m.q;
+    fm.qe = d.qeqe[0];
+    fm.near2 = near2;
+    fm.rm2 = rm * rm;
     if (!CELLS) {
-        for (int b = 32 * part; b < d.N; b += 32 * nparts) {   // warp-uniform trip count
-            const int j = b + lane;
-            const bool v = j < d.N && j != m.i;
-            const int4 p = v ? d.pos4[j] : make_int4(0, 0, 0, 0);
-            const int t = v ? d.ptype[j] : 0;
-            eb_push<CELLS>(v && eb_in_reach(p, m, d), p, j, t, qn, qp, qm, m, d, accf, accd);
+        const int N = d.N, step = 32 * nparts;
+        for (int b = 32 * part; b < N; b += 32 * step) {
+            const int left = nparts == 1 ? (N - b + 31) >> 5 : (N - b + step - 1) / step;
+            eb_screen<CELLS>(b, step, min(left, 32), q, fm, which, w, d);
         }
-        eb_flush<CELLS>(qn, qp, qm, m, d, accf, accd);
         return;
     }
     // The stencil: the cells around the old cell, widened by one along each
     // axis where the particle changed cells (at most 4 x 4 x 4). Lane c (and
     // c + 32) takes stencil cell c: it drops the cell when no point of the
     // cell box lies within reach of the old or the new position, so that the
-    // cell's particles cannot contribute, and the warp's prefix sum over the
-    // remaining cells' counts flattens their slots into one candidate list,
-    // which the warp then screens 32 candidates at a time with all lanes busy.
-    int co[3], cn[3], lo[3], len[3];
-    co[0] = m.co % d.nc[0]; co[1] = (m.co / d.nc[0]) % d.nc[1]; co[2] = m.co / (d.nc[0] * d.nc[1]);
-    cn[0] = m.cn % d.nc[0]; cn[1] = (m.cn / d.nc[0]) % d.nc[1]; cn[2] = m.cn / (d.nc[0] * d.nc[1]);
+    // cell's particles cannot contribute; the remaining cells' batches are
+    // listed by the warp's prefix sum over their numbers.
+    int lo[3], len[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
-        int delta = cn[a] - co[a];
+        // cell_of's coordinate
+        const int co = (int)__umulhi((uint32_t)fm.ho[a] + 0x80000000u, (uint32_t)d.nc[a]);
+        const int cn = (int)__umulhi((uint32_t)fm.hn[a] + 0x80000000u, (uint32_t)d.nc[a]);
+        int delta = cn - co;
         if (delta > 1) delta -= d.nc[a];
         if (delta < -1) delta += d.nc[a];
         if ((delta > 1 || delta < -1) && lane == 0) atomicOr(&d.sc->error, kErrStencil);
-        lo[a] = co[a] + min(delta, 0) - 1;
+        lo[a] = co + min(delta, 0) - 1;
         len[a] = 3 + (delta != 0 ? 1 : 0);
     }
     const int ncell = len[0] * len[1] * len[2];   // <= 64
@@ -258,10 +460,10 @@ __device__ __forceinline__ void eb_pairs_warp(const Move &m, const SysDesc &d, c
     // old plus the minimum-image step, so that both lie on the stencil's side
     // of the box edge); a small margin covers the float rounding of the box
     // bounds (units of 2^32 / L carry ~2^8 units of rounding here)
-    const float reach2m = d.reach2 * 1.0001f + 1e-3f;
-    float uo[3], un[3];
+    float uo[3], un[3], W[3];
 #pragma unroll
     for (int a = 0; a < 3; a++) {
+        W[a] = 4294967296.0f / (float)d.nc[a];
         uo[a] = (float)((uint32_t)m.ho[a] + 0x80000000u);
         un[a] = uo[a] + (float)(int)(m.hn[a] - m.ho[a]);
     }
@@ -272,26 +474,28 @@ __device__ __forceinline__ void eb_pairs_warp(const Move &m, const SysDesc &d, c
         cidv[h] = 0;
         cntv[h] = 0;
         if (c < ncell) {
-            const int i0 = c % len[0], i1 = (c / len[0]) % len[1], i2 = c / (len[0] * len[1]);
+            // by lengths of 3 or 4: c 171 >> 9 is c / 3 for c < 128
+            const int c1 = len[0] == 4 ? c >> 2 : c * 171 >> 9, i0 = c - c1 * len[0];
+            const int i2 = len[1] == 4 ? c1 >> 2 : c1 * 171 >> 9, i1 = c1 - i2 * len[1];
             const int cu[3] = {lo[0] + i0, lo[1] + i1, lo[2] + i2};
             float d2o = 0.0f, d2n = 0.0f;
-            int w[3];
+            int cw[3];
 #pragma unroll
             for (int a = 0; a < 3; a++) {
-                const float W = 4294967296.0f / (float)d.nc[a];
-                const float A = (float)cu[a] * W, B = A + W;
+                const float A = (float)cu[a] * W[a], B = A + W[a];
                 const float xo = fmaxf(fmaxf(A - uo[a], uo[a] - B), 0.0f) * d.s32[a];
                 const float xn = fmaxf(fmaxf(A - un[a], un[a] - B), 0.0f) * d.s32[a];
                 d2o = fmaf(xo, xo, d2o);
                 d2n = fmaf(xn, xn, d2n);
-                w[a] = cu[a] + (cu[a] < 0 ? d.nc[a] : 0) - (cu[a] >= d.nc[a] ? d.nc[a] : 0);
+                cw[a] = cu[a] + (cu[a] < 0 ? d.nc[a] : 0) - (cu[a] >= d.nc[a] ? d.nc[a] : 0);
             }
-            cidv[h] = (w[2] * d.nc[1] + w[1]) * d.nc[0] + w[0];
+            cidv[h] = (cw[2] * d.nc[1] + cw[1]) * d.nc[0] + cw[0];
             if (fminf(d2o, d2n) <= reach2m) cntv[h] = s.ccount[cidv[h]];
         }
     }
-    // inclusive prefix sums of the two halves; start = exclusive
-    int inc0 = cntv[0], inc1 = cntv[1];
+    // inclusive prefix sums of the batches of the two halves
+    const int nb0 = (cntv[0] + 31) >> 5, nb1 = (cntv[1] + 31) >> 5;
+    int inc0 = nb0, inc1 = nb1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int v0 = __shfl_up_sync(0xffffffffu, inc0, o), v1 = __shfl_up_sync(0xffffffffu, inc1, o);
@@ -301,41 +505,23 @@ __device__ __forceinline__ void eb_pairs_warp(const Move &m, const SysDesc &d, c
         }
     }
     const int tot0 = __shfl_sync(0xffffffffu, inc0, 31);
-    const int st0 = inc0 - cntv[0], st1 = tot0 + inc1 - cntv[1];
     const int total = tot0 + __shfl_sync(0xffffffffu, inc1, 31);
-    // screening against the midpoint hm of the step: a partner within reach
-    // of the old or the new position lies within reach + |d|/2 of hm
-    const int hm[3] = {m.ho[0] + ((int)(m.hn[0] - m.ho[0]) >> 1), m.ho[1] + ((int)(m.hn[1] - m.ho[1]) >> 1),
-                       m.ho[2] + ((int)(m.hn[2] - m.ho[2]) >> 1)};
-    const float hd = 0.5f * sqrtf(fmaf(m.dxf[0], m.dxf[0], fmaf(m.dxf[1], m.dxf[1], m.dxf[2] * m.dxf[2])));
-    const float rm = sqrtf(reach2m) + hd + 1e-3f, rm2 = rm * rm;
-    int c = 0;   // warp-uniform: the cell holding candidate b
-    for (int b = 32 * part; b < total; b += 32 * nparts) {
-        // the first stencil cell whose slots reach past b
-        while (true) {
-            const int e = (c < 32 ? __shfl_sync(0xffffffffu, st0, c) + __shfl_sync(0xffffffffu, cntv[0], c)
-                                  : __shfl_sync(0xffffffffu, st1, c - 32) + __shfl_sync(0xffffffffu, cntv[1], c - 32));
-            if (e > b) break;
-            c++;
+    // this part's: batches part, part + nparts, ...
+    const int mine = nparts == 1 ? total : (total - part + nparts - 1) / nparts;
+    const int st0 = inc0 - nb0 - part, st1 = tot0 + inc1 - nb1 - part;
+    const int at0 = nparts == 1 ? st0 : (st0 + nparts - 1) / nparts, at1 = nparts == 1 ? st1 : (st1 + nparts - 1) / nparts;
+    for (int w0 = 0; w0 < mine; w0 += kEbBatch) {   // warp-uniform
+        __syncwarp();
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            int at = (h ? at1 : at0) - w0;
+            for (int x = (h ? at1 * nparts - st1 : at0 * nparts - st0); x < (h ? nb1 : nb0); x += nparts, at++)
+                if (at >= 0 && at < kEbBatch) q.bat[at] = make_int2(cidv[h] * d.cap + 32 * x, cntv[h] - 32 * x);
         }
-        const int g = b + lane;
-        int mc = c;
-        for (int cc = c + 1; cc < ncell; cc++) {   // warp-uniform
-            const int sc0 = cc < 32 ? __shfl_sync(0xffffffffu, st0, cc) : __shfl_sync(0xffffffffu, st1, cc - 32);
-            if (sc0 > b + 31) break;
-            if (sc0 <= g) mc = cc;
-        }
-        const int sA = __shfl_sync(0xffffffffu, st0, mc & 31), sB = __shfl_sync(0xffffffffu, st1, mc & 31);
-        const int cA = __shfl_sync(0xffffffffu, cidv[0], mc & 31), cB = __shfl_sync(0xffffffffu, cidv[1], mc & 31);
-        const int cid = mc < 32 ? cA : cB, slot = g - (mc < 32 ? sA : sB);
-        const bool in = g < total;
-        const int idx = cid * d.cap + slot;
-        const int pid = in ? d.cell_pid[idx] : -1;
-        const int4 pos = in ? d.cell_pos[idx] : make_int4(0, 0, 0, 0);
-        const bool v = pid >= 0 && (pid & 0xFFFFFF) != m.i && dist2(pos, hm[0], hm[1], hm[2], d) <= rm2;
-        eb_push<CELLS>(v, pos, idx, pid >> 24, qn, qp, qm, m, d, accf, accd);
+        __syncwarp();
+        const int n = min(mine - w0, kEbBatch);
+        for (int b = 0; b < n; b += 32) eb_screen<CELLS>(b, 0, min(n - b, 32), q, fm, which, w, d);
     }
-    eb_flush<CELLS>(qn, qp, qm, m, d, accf, accd);
 }
 
 // dU of trial m from one partner at high words p (charge bits in .w), type t,
@@ -532,6 +718,29 @@ __device__ __noinline__ bool eb_rebuild(const SysDesc &d, const EbSmem &s, df &c
     return anybad != 0;
 }
 
+// One item's differences over ng accepted trials (L values of n; the entries a
+// shorter item reads past its own are dropped by the caller).
+template <int L>
+__device__ __forceinline__ void cq_pass(const float4 *tab, int T, const float *qg, int ng, int ix, int iy, int iz,
+                                        unsigned da[kRbLen], unsigned dr[kRbLen], unsigned db[kRbLen],
+                                        unsigned dc[kRbLen]) {
+#pragma unroll 2
+    for (int g = 0; g < ng; g++) {
+        const float4 *e = tab + g * T;
+        const float q2g = qg[g];
+        const float4 ex = e[ix], ey = e[iy];
+        const float2 wn = qk_w(q2g, make_float2(ex.x, ex.y), make_float2(ey.x, ey.y));
+        const float2 wo = qk_w(q2g, make_float2(ex.z, ex.w), make_float2(ey.z, ey.w));
+#pragma unroll
+        for (int u = 0; u < L; u++) {
+            const float4 z = e[iz + u];
+            da[u] += qk_rint_bits(wn.x, z.x) - qk_rint_bits(wo.x, z.z);
+            dr[u] += qk_rint_bits(wn.y, z.y) - qk_rint_bits(wo.y, z.w);
+            db[u] += qk_rint_bits(wn.x, z.y) - qk_rint_bits(wo.x, z.w);
+            dc[u] += qk_rint_bits(wn.y, z.x) - qk_rint_bits(wo.y, z.z);
+        }
+    }
+}
 // Q(k) after a block: every accepted trial a adds c_k(new_a) - c_k(old_a)
 // (ewald.h:665-705). Threads qt = 0..nq-1 (warps 1.. of the CTA, which
 // synchronise among themselves on named barrier 1) own the rebuild's items
@@ -578,22 +787,11 @@ __device__ __noinline__ void eb_commit_qk(const SysDesc &d, const EbSmem &s, uin
             unsigned da[kRbLen], dr[kRbLen], db[kRbLen], dc[kRbLen];
 #pragma unroll
             for (int u = 0; u < kRbLen; u++) da[u] = dr[u] = db[u] = dc[u] = 0u;
-            for (int g = 0; g < ng; g++) {
-                const float4 *e = tab + g * T;
-                const float q2g = qg[g0 + g];
-                const float4 ex = e[ix], ey = e[iy];
-                const float2 wn = qk_w(q2g, make_float2(ex.x, ex.y), make_float2(ey.x, ey.y));
-                const float2 wo = qk_w(q2g, make_float2(ex.z, ex.w), make_float2(ey.z, ey.w));
-#pragma unroll
-                for (int u = 0; u < kRbLen; u++) {
-                    if (u < len) {
-                        const float4 z = e[iz + u];
-                        da[u] += qk_rint_bits(wn.x, z.x) - qk_rint_bits(wo.x, z.z);
-                        dr[u] += qk_rint_bits(wn.y, z.y) - qk_rint_bits(wo.y, z.w);
-                        db[u] += qk_rint_bits(wn.x, z.y) - qk_rint_bits(wo.x, z.w);
-                        dc[u] += qk_rint_bits(wn.y, z.x) - qk_rint_bits(wo.y, z.z);
-                    }
-                }
+            switch (__reduce_max_sync(__activemask(), len)) {   // items are sorted by length
+                case 1: cq_pass<1>(tab, T, qg + g0, ng, ix, iy, iz, da, dr, db, dc); break;
+                case 2: cq_pass<2>(tab, T, qg + g0, ng, ix, iy, iz, da, dr, db, dc); break;
+                case 3: cq_pass<3>(tab, T, qg + g0, ng, ix, iy, iz, da, dr, db, dc); break;
+                default: cq_pass<4>(tab, T, qg + g0, ng, ix, iy, iz, da, dr, db, dc); break;
             }
 #pragma unroll
             for (int u = 0; u < kRbLen; u++) {
@@ -706,7 +904,7 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
     const SysDesc &d = sd;
     EbSmem s = eb_carve(eb_smem_raw, d, CELLS);
     SysScalars *sc = d.sc;
-    // the work split (16 threads per trial, two Gram k-steps per warp) is
+    // the work split (16 threads per trial in the sums, two walks a warp) is
     // written for exactly kEbThreads threads; a cluster must match the
     // system's k-vector split (the same for every CTA of the cluster)
     if (blockDim.x != kEbThreads || (CLUSTER ? C != d.eb_ctas || C > kEbMaxCluster : d.eb_ctas != 1)) {
@@ -734,14 +932,18 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
         s.b.kpack[k] = d.kpack[k0 + k];
         s.b.qfix[k] = q;
     }
-    // 2 pi / L per axis: k.d = sum_a n_a (2 pi / L_a) d_a
-    const float tpl[3] = {6.283185307179586f / d.L[0], 6.283185307179586f / d.L[1], 6.283185307179586f / d.L[2]};
+    // pi / L per axis: k.d / 2 = sum_a n_a (pi / L_a) d_a
+    const float hpl[3] = {3.141592653589793f / d.L[0], 3.141592653589793f / d.L[1], 3.141592653589793f / d.L[2]};
     if (CELLS) {
         const int ncell = d.nc[0] * d.nc[1] * d.nc[2];
         for (int c = tid; c < ncell; c += blockDim.x) s.b.ccount[c] = d.cell_count[c];
         for (int j = tid; j < d.N; j += blockDim.x)
             s.b.pcs[j] = ((uint32_t)d.p_cell[j] << 12) | (uint32_t)d.p_slot[j];
     }
+    // (1.5 sigma)^2 of the largest pair: pair_candidate's careful path (near)
+    float near2 = d.s2[0];
+    for (int t = 1; t < d.n_types * d.n_types; t++) near2 = fmaxf(near2, d.s2[t]);
+    near2 *= 2.25f;
     if (tid < 3) s.Mdf[tid] = make_float2(sc->m[tid][0], sc->m[tid][1]);
     if (CLUSTER) blk_cluster_barrier();   // every CTA of the cluster runs before any remote store
     else __syncthreads();
@@ -759,82 +961,89 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
     // gt + 4 of the step (eb_gram_regs)
     const int gq = lane >> 2, gt = lane & 3, gh = gt & 1, gk = gt >> 1;
     // per-trial records of the k-space phase (in the increment buffer, past
-    // the real-space queues): {d 2pi/L, q eff}, {old high words, fast}, {new high words}
-    float4 *rA = reinterpret_cast<float4 *>(reinterpret_cast<char *>(s.delta) + 16384);
+    // the real-space queues): {d pi/L, 2 q eff}, {high words of the step's midpoint, fast}
+    float4 *rA = reinterpret_cast<float4 *>(reinterpret_cast<char *>(s.delta) + kEbRecords);
     int4 *rB = reinterpret_cast<int4 *>(rA + kEbTrials);
-    int4 *rC = rB + kEbTrials;
+    Trial next{};
+    if (warp == 0 && cur + lane < stop) next = d.trials[cur + lane];
     while (cur < stop) {
         const int kb = (int)((stop - cur) < (int64_t)kEbTrials ? (stop - cur) : (int64_t)kEbTrials);
         // ---- trials of the block (old coordinates: the block start)
-        if (tid < kb) {
-            const Trial tr = d.trials[cur + tid];
-            int64_t xo[3], xn[3];
-#pragma unroll
-            for (int a = 0; a < 3; a++) {
-                xo[a] = d.pos64[3 * tr.idx + a];
-                xn[a] = (int64_t)((uint64_t)xo[a] + (uint64_t)tr.d[a]);
-            }
-            Move m;
-            move_setup(m, tr.idx, xo, xn, __int_as_float(d.pos4[tr.idx].w), d.ptype[tr.idx], d);
-            s.mv[tid] = m;
-            df thr = {tr.thr_hi, tr.thr_lo};
-            if (d.kT != 1.0f) thr = dfm_f(thr, d.kT);
-            s.thr[tid] = make_float2(thr.hi, thr.lo);
-        }
-        __syncthreads();
-        if (tid < kb) {
-            uint32_t c = 0;
-            const int i = s.mv[tid].i;
-            for (int a = 0; a < tid; a++)
-                if (s.mv[a].i == i) c |= 1u << a;
-            s.col[tid] = c;
-        }
-        if (tid < kEbTrials) {
+        if (warp == 0) {   // lane m: trial m
             float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            int4 b = make_int4(0, 0, 0, 1), c = make_int4(0, 0, 0, 0);
-            if (tid < kb) {
-                const Move &M = s.mv[tid];
-                a = make_float4(M.dxf[0] * tpl[0], M.dxf[1] * tpl[1], M.dxf[2] * tpl[2], M.q * d.eff[M.ti]);
-                // |k.d| <= kcc (|d_x| + |d_y| + |d_z|) 2pi/L: within the Taylor
-                // range of expm1_i_horner every k takes the branch-free path
-                const bool fast = (float)d.kcc * (fabsf(a.x) + fabsf(a.y) + fabsf(a.z)) <= 1.6f;
-                b = make_int4(M.ho[0], M.ho[1], M.ho[2], fast ? 1 : 0);
-                c = make_int4(M.hn[0], M.hn[1], M.hn[2], 0);
+            int4 b = make_int4(0, 0, 0, 1);
+            int i = -1 - lane;
+            if (lane < kb) {
+                const Trial tr = next;   // loaded when the previous block was resolved
+                int64_t xo[3], xn[3];
+#pragma unroll
+                for (int x = 0; x < 3; x++) {
+                    xo[x] = d.pos64[3 * tr.idx + x];
+                    xn[x] = (int64_t)((uint64_t)xo[x] + (uint64_t)tr.d[x]);
+                }
+                Move m;
+                move_setup(m, tr.idx, xo, xn, __int_as_float(d.pos4[tr.idx].w), d.ptype[tr.idx], d);
+                s.mv[lane] = m;
+                i = m.i;
+                df thr = {tr.thr_hi, tr.thr_lo};
+                if (d.kT != 1.0f) thr = dfm_f(thr, d.kT);
+                s.thr[lane] = make_float2(thr.hi, thr.lo);
+                a = make_float4(m.dxf[0] * hpl[0], m.dxf[1] * hpl[1], m.dxf[2] * hpl[2], 2.0f * m.q * d.eff[m.ti]);
+                // |k.d| / 2 <= kcc (|d_x| + |d_y| + |d_z|) pi/L: within the Taylor
+                // range of eb_sin every k takes the branch-free path
+                const bool fast = (float)d.kcc * (fabsf(a.x) + fabsf(a.y) + fabsf(a.z)) <= 0.8f;
+                b = make_int4(m.ho[0] + ((int)(m.hn[0] - m.ho[0]) >> 1), m.ho[1] + ((int)(m.hn[1] - m.ho[1]) >> 1),
+                              m.ho[2] + ((int)(m.hn[2] - m.ho[2]) >> 1), fast ? 1 : 0);
             }
-            rA[tid] = a;
-            rB[tid] = b;
-            rC[tid] = c;
+            s.col[lane] = __match_any_sync(0xffffffffu, i) & ((1u << lane) - 1u);   // earlier trials on its particle
+            rA[lane] = a;
+            rB[lane] = b;
         }
         // the k-space records are the last shared input of the phases below:
         // from here each warp runs its corrections, its real-space walks and
         // its k-steps back to back, with no barrier between them (a warp
         // done walking early starts on k space)
         __syncthreads();
-        // ---- real-space and surface corrections c(a, m), a < m (cluster: a
-        // 1/C share per CTA, into CTA 0's table)
-        const int e_lo = CLUSTER ? rank * (kEbTrials * kEbTrials / C) : 0;
-        const int e_hi = CLUSTER ? e_lo + kEbTrials * kEbTrials / C : kEbTrials * kEbTrials;
-        for (int e = e_lo + tid; e < e_hi; e += blockDim.x) {
-            const int a = e / kEbTrials, m = e - a * kEbTrials;
-            float2 out = make_float2(0.0f, 0.0f);
-            if (a < m && m < kb && s.mv[a].i != s.mv[m].i) {
+        // ---- real-space and surface corrections c(a, m), a < m: the
+        // kb (kb - 1) / 2 pairs (cluster: a 1/C share per CTA, into CTA 0's
+        // table), two lanes each, one for a's new and one for its old position
+        {
+            const int np = 2 * ((kb * (kb - 1) / 2 + C - 1 - rank) / C);
+            for (int ub = warp * 32; ub < np; ub += blockDim.x) {   // warp-uniform
+                const int u = ub + lane;
+                df v = {0.0f, 0.0f};
+                int a = 0, m = 0;
+                if (u < np) {
+                    const int e = (u >> 1) * C + rank;
+                    m = (int)((1.0f + sqrtf(8.0f * (float)e + 1.0f)) * 0.5f);
+                    if (m * (m - 1) / 2 > e) m--;
+                    if ((m + 1) * m / 2 <= e) m++;
+                    a = e - m * (m - 1) / 2;
+                }
                 const Move &A = s.mv[a];
                 const Move &Mm = s.mv[m];
-                const int4 pn = make_int4(A.hn[0], A.hn[1], A.hn[2], __float_as_int(A.q));
-                const int4 po = make_int4(A.ho[0], A.ho[1], A.ho[2], __float_as_int(A.q));
-                const short4 en = make_short4((short)A.en[0], (short)A.en[1], (short)A.en[2], 0);
-                const short4 eo = make_short4((short)A.eo[0], (short)A.eo[1], (short)A.eo[2], 0);
-                df c = df_add(eb_pair(Mm, pn, A.ti, &en, d), df_neg(eb_pair(Mm, po, A.ti, &eo, d)));
-                if (d.surf_c != 0.0f) {
-                    float da[3], dm[3];
-                    eb_dM(A, d, da);
-                    eb_dM(Mm, d, dm);
-                    c = df_add_f(c, 2.0f * d.surf_c * fmaf(da[0], dm[0], fmaf(da[1], dm[1], da[2] * dm[2])));
+                if (u < np && A.i != Mm.i) {
+                    const bool old = u & 1;
+                    const int4 pj = make_int4(old ? A.ho[0] : A.hn[0], old ? A.ho[1] : A.hn[1], old ? A.ho[2] : A.hn[2],
+                                              __float_as_int(A.q));
+                    const short4 ext = make_short4((short)(old ? A.eo[0] : A.en[0]), (short)(old ? A.eo[1] : A.en[1]),
+                                                   (short)(old ? A.eo[2] : A.en[2]), 0);
+                    v = eb_pair(Mm, pj, A.ti, &ext, d);
+                    if (!old && d.surf_c != 0.0f) {
+                        float da[3], dm[3];
+                        eb_dM(A, d, da);
+                        eb_dM(Mm, d, dm);
+                        v = df_add_f(v, 2.0f * d.surf_c * fmaf(da[0], dm[0], fmaf(da[1], dm[1], da[2] * dm[2])));
+                    }
                 }
-                out = make_float2(c.hi, c.lo);
+                const df w = {__shfl_xor_sync(0xffffffffu, v.hi, 1), __shfl_xor_sync(0xffffffffu, v.lo, 1)};
+                if (u < np && !(u & 1)) {
+                    const df c = df_add(v, df_neg(w));
+                    float2 *to = &s.corr[a * kEbTrials + m];
+                    if (CLUSTER) eb_st_remote(to, 0, make_float2(c.hi, c.lo));
+                    else *to = make_float2(c.hi, c.lo);
+                }
             }
-            if (CLUSTER) eb_st_remote(&s.corr[e], 0, out);
-            else s.corr[e] = out;
         }
         // ---- real-space base: warp w sums trials w, w + nwarp, ...; its
         // candidate queue lives in the (not yet used) increment buffer. On a
@@ -843,19 +1052,31 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
         {
             const int P = CLUSTER ? (C + 1) / 2 : 1;
             const int u0 = CLUSTER ? rank * nwarp + warp : warp, du = CLUSTER ? C * nwarp : nwarp;
-            for (int u = u0; u < kb * P; u += du) {
-                const int m = u / P, part = u - m * P;
-                const Move mv = s.mv[m];
-                float accf = 0.0f;
-                df accd = {0.0f, 0.0f};
-                int4 *qp = reinterpret_cast<int4 *>(s.delta) + warp * 48;
-                int2 *qm = reinterpret_cast<int2 *>(qp + 32);
-                eb_pairs_warp<CELLS>(mv, d, s.b, qp, qm, part, P, accf, accd);
-                const df p = warp_sum_df(df_add_f(accd, accf));
-                if (lane == 0) {
-                    if (CLUSTER) eb_st_remote(&s.xreal[m * P + part], 0, make_float2(p.hi, p.lo));
-                    else s.partR[m] = make_float2(p.hi, p.lo);
-                }
+            EbQueue q = eb_queue(reinterpret_cast<char *>(s.delta) + warp * kEbQueueBytes);
+            EbWalk w{{s.mv + min(u0 / P, kb - 1), s.mv + min((u0 + du) / P, kb - 1)}, 0.0f, {0.0f, 0.0f}, {0.0f, 0.0f}};
+            float f0 = 0.0f;   // at most two walks a warp: kb P <= 2 du
+#pragma unroll 1
+            for (int h = 0; h < 2; h++) {
+                const int u = u0 + h * du;
+                f0 = h ? w.f : 0.0f;
+                w.f = 0.0f;
+                if (u < kb * P) eb_pairs_warp<CELLS>(h, w, d, s.b, q, near2, u % P, P);
+            }
+            eb_flush_near<CELLS>(q, w, d);
+            // both sums in one tree, the half-warps exchanging first
+            const df p0 = df_add_f(w.a0, f0), p1 = df_add_f(w.a1, w.f);
+            const bool hi = lane >= 16;
+            df v = hi ? p1 : p0;
+            const df o = hi ? p0 : p1;
+            v = df_add(v, df{__shfl_xor_sync(0xffffffffu, o.hi, 16), __shfl_xor_sync(0xffffffffu, o.lo, 16)});
+#pragma unroll
+            for (int x = 8; x > 0; x >>= 1)
+                v = df_add(v, df{__shfl_xor_sync(0xffffffffu, v.hi, x), __shfl_xor_sync(0xffffffffu, v.lo, x)});
+            const int u = u0 + (lane >> 4) * du;
+            if ((lane & 15) == 0 && u < kb * P) {
+                const float2 p = make_float2(v.hi, v.lo);
+                if (CLUSTER) eb_st_remote(&s.xreal[u], 0, p);
+                else s.partR[u] = p;
             }
         }
         // ---- reciprocal base and Gram matrix. Lane (gq, gt) and its partner
@@ -884,25 +1105,21 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
                     const int t = gq + 8 * (2 * gh + rr);
                     const float4 a = rA[t];
                     const int4 b = rB[t];
-                    const int ho[3] = {b.x, b.y, b.z};
-                    const uint32_t ph = phase(nx, ny, nz, ho);
-                    const float2 e = sincos_turns(ph, s.b.sc_tab);
-                    const float phi = fmaf(fx, a.x, fmaf(fy, a.y, fz * a.z));
-                    float2 w;
-                    if (b.w || fabsf(phi) <= 1.6f) {
-                        w = expm1_i_horner(phi);
-                    } else {
-                        const int4 c = rC[t];
-                        const int hn[3] = {c.x, c.y, c.z};
-                        const float2 en = sincos_turns(phase(nx, ny, nz, hn) - ph, s.b.sc_tab);
-                        w = make_float2(en.x - 1.0f, en.y);
+                    // D = q (e^{ik.r_new} - e^{ik.r_old}) = 2 q sin(k.d / 2) i e^{ik.r_mid}
+                    const int hm[3] = {b.x, b.y, b.z};
+                    float2 e = sincos_turns(phase(nx, ny, nz, hm), s.b.sc_tab);
+                    const float half = fmaf(fx, a.x, fmaf(fy, a.y, fz * a.z));
+                    float sn = eb_sin(half);
+                    if (!b.w && fabsf(half) > 0.8f) {   // a long step: both angles from the exact phases
+                        const Move &M = s.mv[t];
+                        const uint32_t po = phase(nx, ny, nz, M.ho);
+                        const int32_t hp = (int32_t)(phase(nx, ny, nz, M.hn) - po) >> 1;
+                        e = sincos_turns(po + (uint32_t)hp, s.b.sc_tab);
+                        sn = sincos_turns((uint32_t)hp, s.b.sc_tab).y;
                     }
-                    const float live = kraw < K ? a.w : 0.0f;   // q eff; 0 past K and for idle trials
-                    float2 dd = cmul(e, w);
-                    dd.x *= live;
-                    dd.y *= live;
-                    kac[rr] = fmaf(kv.x, fmaf(2.0f, fmaf(kv.y, dd.x, kv.z * dd.y), fmaf(dd.x, dd.x, dd.y * dd.y)),
-                                   kac[rr]);
+                    const float amp = (kraw < K ? a.w : 0.0f) * sn;   // 0 past K and for idle trials
+                    const float2 dd = make_float2(-amp * e.y, amp * e.x);
+                    kac[rr] = fmaf(kv.x, fmaf(2.0f, fmaf(kv.y, dd.x, kv.z * dd.y), amp * amp), kac[rr]);
                     const float own = (gh ? dd.y : dd.x) * kv.w, other = (gh ? dd.x : dd.y) * kv.w;
                     const float recv = __shfl_xor_sync(0xffffffffu, other, 1);
                     xf[rr][j] = gh ? recv : own;
@@ -929,15 +1146,26 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
                 for (int x = 0; x < 6; x++)
                     *reinterpret_cast<float4 *>(q + x * 128) = make_float4(gc[x][0], gc[x][1], gc[x][2], gc[x][3]);
             }
-            if (tid < kEbTrials) {
-                // trial t = gq' + 8 r': lanes gq' * 4 + (r' >> 1) + 2 gk', slot rr = r' & 1
-                const int tq = tid & 7, tr = tid >> 3;
-                df v = {0.0f, 0.0f};
-                for (int w = 0; w < nw; w++)
-                    for (int g2 = 0; g2 < 2; g2++)
-                        v = df_add_f(v, KP[(w * 32 + tq * 4 + (tr >> 1) + 2 * g2) * 2 + (tr & 1)]);
-                if (CLUSTER) eb_st_remote(&s.xkbase[rank * kEbTrials + tid], 0, make_float2(v.hi, v.lo));
-                else s.kbase[tid] = make_float2(v.hi, v.lo);
+            {
+                // warp w sums trials w and w + 16 over their 32 partials (16
+                // warps, gk' = 0, 1) in one tree, the half-warps exchanging
+                // first. Trial t = gq' + 8 r': lanes gq' * 4 + (r' >> 1) + 2 gk',
+                // slot rr = r' & 1
+                auto part = [&](int t) {
+                    const int tq = t & 7, tr = t >> 3;
+                    return KP[((lane >> 1) * 32 + tq * 4 + (tr >> 1) + 2 * (lane & 1)) * 2 + (tr & 1)];
+                };
+                const float p0 = part(warp), p1 = part(warp + 16);
+                const bool hi = lane >= 16;
+                df v = two_sum(hi ? p1 : p0, __shfl_xor_sync(0xffffffffu, hi ? p0 : p1, 16));
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1)
+                    v = df_add(v, df{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)});
+                if ((lane & 15) == 0) {
+                    const int t = warp + lane;
+                    if (CLUSTER) eb_st_remote(&s.xkbase[rank * kEbTrials + t], 0, make_float2(v.hi, v.lo));
+                    else s.kbase[t] = make_float2(v.hi, v.lo);
+                }
             }
             __syncthreads();
             if (warp >= nw / 2) {
@@ -986,19 +1214,19 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
                     const df cs = df_add_f(df{c.x, c.y}, 2.0f * v);
                     s.corr[row * kEbTrials + col] = make_float2(cs.hi, cs.lo);
                 }
-                if (tid < kEbTrials) {
-                    const int P = (C + 1) / 2;
-                    df kv = {0.0f, 0.0f}, rv = {0.0f, 0.0f};
-                    for (int r = 0; r < C; r++) {
-                        const float2 x = s.xkbase[r * kEbTrials + tid];
-                        kv = df_add(kv, df{x.x, x.y});
-                    }
-                    for (int p = 0; p < P; p++) {
-                        const float2 x = s.xreal[tid * P + p];
-                        rv = df_add(rv, df{x.x, x.y});
-                    }
-                    s.kbase[tid] = make_float2(kv.hi, kv.lo);
-                    s.partR[tid] = make_float2(rv.hi, rv.lo);
+                // 16 threads per trial: one per rank and part, in one tree each
+                const int t = tid >> 4, r = tid & 15, P = (C + 1) / 2;
+                const float2 x = r < C ? s.xkbase[r * kEbTrials + t] : make_float2(0.0f, 0.0f);
+                const float2 y = r < P && t < kb ? s.xreal[t * P + r] : make_float2(0.0f, 0.0f);
+                df kv = {x.x, x.y}, rv = {y.x, y.y};
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) {
+                    kv = df_add(kv, df{__shfl_xor_sync(0xffffffffu, kv.hi, o), __shfl_xor_sync(0xffffffffu, kv.lo, o)});
+                    rv = df_add(rv, df{__shfl_xor_sync(0xffffffffu, rv.hi, o), __shfl_xor_sync(0xffffffffu, rv.lo, o)});
+                }
+                if (r == 0) {
+                    s.kbase[t] = make_float2(kv.hi, kv.lo);
+                    s.partR[t] = make_float2(rv.hi, rv.lo);
                 }
             }
         }
@@ -1017,40 +1245,40 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
             const float2 th = lane < kb ? s.thr[lane] : make_float2(0.0f, 0.0f);
             uint32_t accm = 0;
             int done = kb;
+            // NonbondedEwald::update (ewald.h:633): a rebuild after
+            // update_frequency accepted trials ends the block there
+            const int every = max(uf, 1), left = d.skip_rebuild ? 64 : max(every - cnt_acc, 1);
+            const bool due = left <= kb;   // a rebuild may fall due in this block
+            float2 cn = s.corr[lane];
             for (int a = 0; a < kb; a++) {
                 // lane a decides: its S already holds the corrections of every
                 // accepted trial before it in the block. Movebase::metropolis
                 // (move.h:567-573): reject iff dU > kT (-ln u); a NaN dU
-                // compares false there: accepted
-                const float2 c = s.corr[a * kEbTrials + lane];   // loaded ahead of the decision
-                // every lane forms its own flags; lane a's are the ones used
-                const bool nan = !(S.hi == S.hi);
-                const int fl = ((colm & accm) != 0u ? 1 : 0) | (nan || !df_gt(S, df{th.x, th.y}) ? 2 : 0) | (nan ? 4 : 0);
-                const int f = __shfl_sync(0xffffffffu, fl, a);
-                if (f & 1) {   // its particle was moved by an accepted trial of this block
+                // compares false there: accepted. Every lane forms its flags and
+                // the sum it would go on with; bit a of their ballots selects, so
+                // a step has no divergent branch
+                const float2 c = cn;
+                cn = s.corr[min(a + 1, kEbTrials - 1) * kEbTrials + lane];
+                const df Sc = df_add_quick(S, df{c.x, c.y});
+                const uint32_t again = __ballot_sync(0xffffffffu, (colm & accm) != 0u);
+                const uint32_t ok = __ballot_sync(0xffffffffu, !df_gt(S, df{th.x, th.y}));
+                if ((again >> a) & 1u) {   // its particle was moved by an accepted trial of this block
                     done = a;
                     break;
                 }
-                if (f & 4) err |= kErrNonFinite;
-                if (f & 2) {
-                    accm |= 1u << a;
-                    nacc++;
-                    const df Sc = df_add_quick(S, df{c.x, c.y});
-                    const bool later = lane > a && lane < kb;
-                    S.hi = later ? Sc.hi : S.hi;
-                    S.lo = later ? Sc.lo : S.lo;
-                    // NonbondedEwald::update (ewald.h:633): a rebuild after
-                    // update_frequency accepted trials ends the block here
-                    if (++cnt_acc > uf - 1) {
-                        cnt_acc = 0;
-                        if (!d.skip_rebuild) {
-                            rebuild = true;
-                            done = a + 1;
-                            break;
-                        }
-                    }
+                accm |= ok & (1u << a);
+                const bool add = ((ok >> a) & 1u) && lane > a;
+                S.hi = add ? Sc.hi : S.hi;
+                S.lo = add ? Sc.lo : S.lo;
+                if (due && __popc(accm) == left) {
+                    rebuild = true;
+                    done = a + 1;
+                    break;
                 }
             }
+            nacc += __popc(accm);
+            cnt_acc = rebuild ? 0 : (cnt_acc + __popc(accm)) % every;
+            if (__any_sync(0xffffffffu, lane < done && !(S.hi == S.hi))) err |= kErrNonFinite;
             // lane m's S is trial m's dU as decided: log it, and add the
             // accepted ones to the running sums (a fixed-order warp sum)
             const bool take = lane < done && ((accm >> lane) & 1u);
@@ -1080,6 +1308,7 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
         const uint32_t accm = (uint32_t)s.info[1];
         rebuild = s.info[2] != 0;
         cnt_acc = s.info[3];
+        if (warp == 0 && cur + done + lane < stop) next = d.trials[cur + done + lane];
         // ---- apply the accepted trials. Warp 0 commits the positions and
         // cell lists while warps 1.. update Q(k), synchronising among
         // themselves on named barrier 1; the block barrier below joins the two.
@@ -1103,18 +1332,18 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
             }
             const uint32_t movers = __ballot_sync(0xffffffffu, mover);
             __syncwarp();   // the lanes' records are visible to lane 0
-            if (lane == 0) {
-                df M[3] = {{s.Mdf[0].x, s.Mdf[0].y}, {s.Mdf[1].x, s.Mdf[1].y}, {s.Mdf[2].x, s.Mdf[2].y}};
-                for (int a = 0; a < done; a++) {
-                    if (!((accm >> a) & 1u)) continue;
-                    if ((movers >> a) & 1u) eb_cell_move(s.mv[a], d, s.b);
-                    float dm[3];
-                    eb_dM(s.mv[a], d, dm);
+            if (lane == 0)
+                for (uint32_t left = movers; left; left &= left - 1) eb_cell_move(s.mv[__ffs(left) - 1], d, s.b);
+            // M: the accepted changes in one tree
+            float dm[3] = {0.0f, 0.0f, 0.0f};
+            if (mine) eb_dM(s.mv[lane], d, dm);
+            df M[3];
 #pragma unroll
-                    for (int x = 0; x < 3; x++) M[x] = df_add_f(M[x], dm[x]);
-                }
-#pragma unroll
-                for (int x = 0; x < 3; x++) s.Mdf[x] = make_float2(M[x].hi, M[x].lo);
+            for (int x = 0; x < 3; x++) M[x] = warp_sum_df(df{dm[x], 0.0f});
+            if (lane < 3) {
+                const df v = lane == 0 ? M[0] : lane == 1 ? M[1] : M[2];
+                const df t = df_add(df{s.Mdf[lane].x, s.Mdf[lane].y}, v);
+                s.Mdf[lane] = make_float2(t.hi, t.lo);
             }
         } else if (tid >= 32 && live) {
             // Q(k) += sum over accepted trials of c_k(new) - c_k(old), over

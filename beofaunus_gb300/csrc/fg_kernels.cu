@@ -99,8 +99,7 @@ __device__ __forceinline__ float rsqrt_nr(float r2) {
 // erfc for x >= 0: the Chebyshev fit of Press, Teukolsky, Vetterling and
 // Flannery (Numerical Recipes in C, 2nd ed., section 6.2, "erfcc"),
 // fractional error below 1.2e-7 everywhere.
-__device__ __forceinline__ float erfc_nr(float z) {
-    const float t = __frcp_rn(fmaf(0.5f, z, 1.0f));
+__device__ __forceinline__ float erfc_nr_at(float t, float z) {   // t = 1 / (1 + z / 2)
     float p = fmaf(t, 0.17087277f, -0.82215223f);
     p = fmaf(t, p, 1.48851587f);
     p = fmaf(t, p, -1.13520398f);
@@ -112,6 +111,7 @@ __device__ __forceinline__ float erfc_nr(float z) {
     p = fmaf(t, p, -1.26551223f);
     return t * expf(fmaf(-z, z, p));
 }
+__device__ __forceinline__ float erfc_nr(float z) { return erfc_nr_at(__frcp_rn(fmaf(0.5f, z, 1.0f)), z); }
 
 // EwaldReal (kappa-screened form, ewald.h:109) + WCA; qq = qa qb QeQe lB.
 // NEAR: correctly rounded sqrt/divide and erfcf for the few pairs close to
