@@ -69,7 +69,7 @@ struct DipTrial {
 
 struct DipScalars {
     int64_t cursor;       // next trial of the staged stream
-    int64_t n_trials;     // end of the stream for this launch
+    int64_t acc0;         // n_accepted when the stream was staged
     int64_t n_accepted;   // cumulative
     int64_t n_rebuilds;   // cumulative Q(k) rebuilds
     int32_t error;
@@ -542,16 +542,38 @@ __global__ void __launch_bounds__(kDipMaxThreads, 1) dip_build_kernel(const DipD
     dip_rebuild(d, A, S, before, after);
 }
 
-// mode 0: run the staged stream [cursor, n_trials) with Metropolis decisions;
+// mode 0: run the staged stream [cursor, end) with Metropolis decisions;
 // mode 1: evaluate trials[0] (explicit) and keep it pending;
 // mode 2: apply the pending trials[0] as accepted.
 // MAXT: the launch bound. 128 threads per system at most 128 registers
 // (four systems, sixteen warps on an SM) or up to kDipMaxThreads at one CTA
 // per SM.
+// The systems of a launch: one, or many by their device descriptors with the
+// ends of their streams (no trial of index cap or above runs).
+struct DipLaunch {
+    const DipDesc *one;
+    const DipDesc *const *many;
+    const int64_t *ends;
+    int64_t end, cap;
+};
+
+// A newly staged stream: cursor, per-stream sum and flags from zero.
+__global__ void dip_begin_kernel(DipScalars *sc) {
+    sc->cursor = 0;
+    sc->acc0 = sc->n_accepted;
+    sc->usum = 0.0;
+    sc->error = 0;
+}
+// The scalars of many systems into one array (one copy to the host).
+__global__ void dip_gather_kernel(DipLaunch l, int n, DipScalars *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = l.many ? *l.many[i]->sc : *l.one->sc;
+}
+
 template <int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(const DipDesc *__restrict__ descs, int mode,
-                                                                               int stage) {
-    const DipDesc &d = descs[blockIdx.x];
+__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(DipLaunch l, int mode, int stage) {
+    const DipDesc *__restrict__ dp = l.many ? l.many[blockIdx.x] : l.one;
+    const DipDesc &d = *dp;
     __shared__ DipShared S;
     extern __shared__ __align__(16) unsigned char dsm[];
     float4 *eyz = reinterpret_cast<float4 *>(dsm);   // df complex
@@ -601,7 +623,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(co
     int64_t t0 = 0, t1 = 1;
     if (mode == 0) {
         t0 = d.sc->cursor;
-        t1 = d.sc->n_trials;
+        t1 = min(l.many ? l.ends[blockIdx.x] : l.end, l.cap);
     }
     DipTrial nxt;   // lanes 0..2: the next trial's record, loaded one trial ahead
     if (tid < 3 && t0 < t1) nxt = d.trials[mode == 0 ? t0 : 0];
@@ -916,8 +938,6 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(co
     if (tid == 0) {
         if (mode == 0) sc.cursor = t1;
         for (int a = 0; a < 6; a++) sc.M[a] = S.M[a];
-        // the host may have moved the stream end while this kernel was queued
-        sc.n_trials = d.sc->n_trials;
         *d.sc = sc;
     }
 }
@@ -976,7 +996,12 @@ struct fg_dipsys {
     int64_t log_cap = 0;
     fgd::DipScalars *sc = nullptr;
     int64_t n_stream = 0;
-    int64_t acc0 = 0;
+    // dip_run's workspace of the system it launches from: n descriptor
+    // pointers, n stream ends, n scalars
+    void *run_ws = nullptr;
+    int run_cap = 0;
+    fgd::DipDesc pushed{};   // what d_desc holds
+    bool has_pushed = false;
     bool pending = false;
     bool state_set = false;
     std::vector<double> ak_h, charges_h, mus_h;
@@ -995,7 +1020,7 @@ void dip_free(fg_dipsys *h) {
     dip_radial_release(h);
     void *ptrs[] = {h->d_desc, h->pos, h->mu, h->mus, h->q, h->ak, h->pairs, h->type, h->nearq, h->pf, h->sctab, h->yzl, h->kn,
                     h->qi, h->qd,
-                    h->fqi, h->fqd, h->dqi, h->dqd, h->akf, h->trials, h->log_du, h->log_acc, h->sc};
+                    h->fqi, h->fqd, h->dqi, h->dqd, h->akf, h->trials, h->log_du, h->log_acc, h->sc, h->run_ws};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -1012,6 +1037,9 @@ int dip_dmalloc(fg_dipsys *h, void **p, size_t bytes) {
 }
 
 int dip_push_desc(fg_dipsys *h) {
+    if (h->has_pushed && !std::memcmp(&h->pushed, &h->desc, sizeof(fgd::DipDesc))) return FG_OK;
+    std::memcpy(&h->pushed, &h->desc, sizeof(fgd::DipDesc));
+    h->has_pushed = true;
     CK(cudaMemcpyAsync(h->d_desc, &h->desc, sizeof(fgd::DipDesc), cudaMemcpyHostToDevice, h->stream));
     return FG_OK;
 }
@@ -1302,7 +1330,7 @@ size_t dip_launch_smem(fg_dipsys *const *sys, int n, int &stage) {
     return stage ? st : yz;
 }
 
-int dip_launch(fg_dipsys *const *sys, const fgd::DipDesc *descs, int n, int mode, cudaStream_t st) {
+int dip_launch(fg_dipsys *const *sys, const fgd::DipLaunch &l, int n, int mode, cudaStream_t st) {
     int stage = 0;
     size_t smem = dip_launch_smem(sys, n, stage);
     if (mode != 0) {
@@ -1313,9 +1341,9 @@ int dip_launch(fg_dipsys *const *sys, const fgd::DipDesc *descs, int n, int mode
     const void *fn = T <= 128 ? (const void *)fgd::dip_sweep_kernel<128> : (const void *)fgd::dip_sweep_kernel<fgd::kDipMaxThreads>;
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (T <= 128)
-        fgd::dip_sweep_kernel<128><<<n, T, smem, st>>>(descs, mode, stage);
+        fgd::dip_sweep_kernel<128><<<n, T, smem, st>>>(l, mode, stage);
     else
-        fgd::dip_sweep_kernel<fgd::kDipMaxThreads><<<n, T, smem, st>>>(descs, mode, stage);
+        fgd::dip_sweep_kernel<fgd::kDipMaxThreads><<<n, T, smem, st>>>(l, mode, stage);
     CK(cudaGetLastError());
     return FG_OK;
 }
@@ -1334,45 +1362,58 @@ int dip_run(fg_dipsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
         CK(cudaStreamSynchronize(h->stream));
     }
     cudaStream_t st = h0->stream;
-    const fgd::DipDesc *descs = h0->d_desc;
-    fgd::DipDesc *tmp = nullptr;
+    // Two copies serve all systems: pointers and stream ends in, scalars out
+    // (8 bytes in and 136 out for each of 608 systems, one at a time, and
+    // their descriptors were 8 ms beside an 18 ms kernel).
+    if (h0->run_cap < n) {
+        const size_t each = sizeof(void *) + sizeof(int64_t) + sizeof(fgd::DipScalars);
+        if (h0->run_ws) cudaFree(h0->run_ws);
+        h0->run_ws = nullptr;
+        h0->device_bytes -= (size_t)h0->run_cap * each;
+        h0->run_cap = 0;
+        int rc = dip_dmalloc(h0, &h0->run_ws, (size_t)n * each);
+        if (rc) return rc;
+        h0->run_cap = n;
+    }
+    fgd::DipScalars *const out = reinterpret_cast<fgd::DipScalars *>((char *)h0->run_ws + (size_t)16 * h0->run_cap);
+    fgd::DipLaunch l{h0->d_desc, nullptr, nullptr, h0->n_stream, 0};
     if (n > 1) {
-        std::vector<fgd::DipDesc> v(n);
-        for (int i = 0; i < n; i++) v[i] = sys[i]->desc;
-        CK(cudaMalloc(&tmp, n * sizeof(fgd::DipDesc)));
-        CK(cudaMemcpyAsync(tmp, v.data(), n * sizeof(fgd::DipDesc), cudaMemcpyHostToDevice, st));
-        descs = tmp;
+        std::vector<int64_t> v(2 * (size_t)n);
+        for (int i = 0; i < n; i++) {
+            v[i] = (int64_t)(intptr_t)sys[i]->d_desc;
+            v[n + i] = sys[i]->n_stream;
+        }
+        CK(cudaMemcpyAsync(h0->run_ws, v.data(), v.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+        l.many = reinterpret_cast<const fgd::DipDesc *const *>(h0->run_ws);
+        l.ends = reinterpret_cast<const int64_t *>(h0->run_ws) + n;
     }
     // launches of at most kChunk trials per system keep each kernel short
     const int64_t kChunk = 16384;
     const int64_t nl = (maxn + kChunk - 1) / kChunk;
-    std::vector<int64_t> ends((size_t)std::max<int64_t>(nl, 1) * n);
     CK(cudaEventRecord(h0->ev0, st));
     int rc = FG_OK;
     for (int64_t c = 0; c < nl && !rc; c++) {
-        for (int i = 0; i < n; i++) {
-            int64_t &e = ends[(size_t)c * n + i];
-            e = std::min(sys[i]->n_stream, (c + 1) * kChunk);
-            CK(cudaMemcpyAsync(&sys[i]->sc->n_trials, &e, sizeof(int64_t), cudaMemcpyHostToDevice, st));
-        }
-        rc = dip_launch(sys, descs, n, 0, st);
+        l.cap = (c + 1) * kChunk;
+        rc = dip_launch(sys, l, n, 0, st);
     }
     CK(cudaEventRecord(h0->ev1, st));
-    CK(cudaEventSynchronize(h0->ev1));
-    if (tmp) cudaFree(tmp);
-    if (rc) return rc;
+    if (rc) {
+        cudaStreamSynchronize(st);
+        return rc;
+    }
+    fgd::dip_gather_kernel<<<(n + 127) / 128, 128, 0, st>>>(l, n, out);
+    CK(cudaGetLastError());
+    std::vector<fgd::DipScalars> s1(n);
+    CK(cudaMemcpyAsync(s1.data(), out, (size_t)n * sizeof(fgd::DipScalars), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
     float ms = 0.0f;
     CK(cudaEventElapsedTime(&ms, h0->ev0, h0->ev1));
-    std::vector<fgd::DipScalars> s1(n);
-    for (int i = 0; i < n; i++)
-        CK(cudaMemcpyAsync(&s1[i], sys[i]->sc, sizeof(fgd::DipScalars), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
     fg_sweep_stats tot{};
     int errs = 0;
     for (int i = 0; i < n; i++) {
         fg_sweep_stats x{};
         x.trials = s1[i].cursor;
-        x.accepted = s1[i].n_accepted - sys[i]->acc0;
+        x.accepted = s1[i].n_accepted - s1[i].acc0;
         x.energy_change = s1[i].usum;
         x.device_ms = ms;
         x.sweep_kernel_ms = ms;
@@ -1436,16 +1477,10 @@ int dip_upload(fg_dipsys *h, int64_t n, const int32_t *kind, const int32_t *idx,
     int rc = dip_ensure_trials(h, n, log);
     if (rc) return rc;
     if (n) CK(cudaMemcpyAsync(h->trials, tr.data(), n * sizeof(fgd::DipTrial), cudaMemcpyHostToDevice, h->stream));
-    fgd::DipScalars s;
-    rc = dip_read_scalars(h, s);
-    if (rc) return rc;
-    s.cursor = 0;
-    s.n_trials = 0;
-    s.usum = 0.0;
-    s.error = 0;
-    h->acc0 = s.n_accepted;
+    fgd::dip_begin_kernel<<<1, 1, 0, h->stream>>>(h->sc);
+    CK(cudaGetLastError());
     h->n_stream = n;
-    return dip_write_scalars(h, s);
+    return FG_OK;
 }
 
 }  // namespace
@@ -1758,7 +1793,7 @@ int fg_dip_trial_du(fg_dipsys *h, int32_t i, const double *new_xyz, const double
     int rc = dip_ensure_trials(h, 1, false);
     if (rc) return rc;
     CK(cudaMemcpyAsync(h->trials, &t, sizeof(t), cudaMemcpyHostToDevice, h->stream));
-    rc = dip_launch(&h, h->d_desc, 1, 1, h->stream);
+    rc = dip_launch(&h, {h->d_desc, nullptr, nullptr, 0, 0}, 1, 1, h->stream);
     if (rc) return rc;
     fgd::DipScalars s;
     rc = dip_read_scalars(h, s);
@@ -1777,7 +1812,7 @@ int fg_dip_commit(fg_dipsys *h, int32_t accepted, double *correction) {
     if (!accepted) return FG_OK;
     fgd::DipScalars s0, s1;
     int rc = dip_read_scalars(h, s0);
-    if (!rc) rc = dip_launch(&h, h->d_desc, 1, 2, h->stream);
+    if (!rc) rc = dip_launch(&h, {h->d_desc, nullptr, nullptr, 0, 0}, 1, 2, h->stream);
     if (!rc) rc = dip_read_scalars(h, s1);
     if (rc) return rc;
     // what update() returns: the reciprocal-energy change of a Q(k) rebuild

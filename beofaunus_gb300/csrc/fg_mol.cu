@@ -96,6 +96,7 @@ struct MolScalars {
     int32_t pad;
     float u_hi, u_lo;        // sum of accepted dU of the current stream
     float utot_hi, utot_lo;  // running total energy
+    int64_t acc0;        // n_accepted when the stream was staged
 };
 
 struct alignas(16) MolDesc {
@@ -1240,6 +1241,20 @@ __global__ void mol_total_kernel(const MolDesc *__restrict__ descs, int chunk, d
     }
 }
 
+// A newly staged stream: cursor, per-stream sum and flags from zero.
+__global__ void mol_begin_kernel(MolScalars *sc, int64_t n) {
+    sc->cursor = 0;
+    sc->n_trials = n;
+    sc->acc0 = sc->n_accepted;
+    sc->u_hi = sc->u_lo = 0.0f;
+    sc->error = 0;
+}
+// The scalars of many systems into one array (one copy to the host).
+__global__ void mol_gather_kernel(const MolDesc *descs, int n, MolScalars *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = *descs[i].sc;
+}
+
 }  // namespace fgm
 
 // ==================================================================== host side
@@ -1270,7 +1285,11 @@ struct fg_molsys {
     double pending_du = 0.0;
     int64_t n_stream = 0;   // trials in the staged stream
     bool staged = false;    // a stream is staged and not yet run (it occupies the trial buffer)
-    int64_t acc0 = 0;       // accepted count when the stream was staged
+    // mol_run's workspace of the system it launches from: 2 n descriptors, n scalars
+    void *run_ws = nullptr;
+    int run_cap = 0;
+    fgm::MolDesc pushed{};  // what d_desc holds
+    bool has_pushed = false;
     bool has_cm = false;
     bool state_set = false;
     std::vector<int32_t> types;
@@ -1297,7 +1316,7 @@ int mol_dmalloc(fg_molsys *h, void **p, size_t bytes) {
 void mol_free(fg_molsys *h) {
     void *ptrs[] = {h->d_desc, h->rep_pos, h->rep_cm, h->rep_mu, h->mus, h->pos4, h->dip_pos4,
                     h->site_dip, h->dip_site, h->dip4, h->trials, h->log_du, h->log_acc, h->sc,
-                    h->expl_pos, h->expl_mu, h->eval_du, h->tot, h->expl_cm};
+                    h->expl_pos, h->expl_mu, h->eval_du, h->tot, h->expl_cm, h->run_ws};
     for (void *p : ptrs)
         if (p) cudaFree(p);
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -1450,6 +1469,9 @@ int mol_alloc_replicas(fg_molsys *h, int C) {
 
 int mol_push_desc(fg_molsys *h) {
     h->desc.C = h->C;
+    if (h->has_pushed && !std::memcmp(&h->pushed, &h->desc, sizeof(fgm::MolDesc))) return FG_OK;
+    std::memcpy(&h->pushed, &h->desc, sizeof(fgm::MolDesc));
+    h->has_pushed = true;
     CK(cudaMemcpyAsync(h->d_desc, &h->desc, sizeof(fgm::MolDesc), cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
     return FG_OK;
@@ -1561,17 +1583,8 @@ int mol_upload(fg_molsys *h, int64_t n, const int32_t *mol, const double *axis, 
     std::vector<fgm::MolTrial> tr;
     mol_make_trials(h, n, mol, axis, angle, center, trans, u, rotate, translate, tr);
     if (n > 0) CK(cudaMemcpyAsync(h->trials, tr.data(), n * sizeof(fgm::MolTrial), cudaMemcpyHostToDevice, h->stream));
-    fgm::MolScalars s0;
-    rc = mol_read_scalars(h, s0);
-    if (rc) return rc;
-    h->acc0 = s0.n_accepted;
-    fgm::MolScalars s = s0;
-    s.cursor = 0;
-    s.n_trials = n;
-    s.u_hi = s.u_lo = 0.0f;
-    s.error = 0;
-    rc = mol_write_scalars(h, s);
-    if (rc) return rc;
+    fgm::mol_begin_kernel<<<1, 1, 0, h->stream>>>(h->sc, n);
+    CK(cudaGetLastError());
     h->n_stream = n;
     h->staged = true;
     h->desc.log_du = log ? h->log_du : nullptr;
@@ -1640,17 +1653,23 @@ int mol_run(fg_molsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
     }
     cudaStream_t st = h0->stream;
     const fgm::MolDesc *descs = h0->d_desc;
-    fgm::MolDesc *tmp = nullptr;
+    if (h0->run_cap < n) {
+        const size_t each = 2 * sizeof(fgm::MolDesc) + sizeof(fgm::MolScalars);
+        if (h0->run_ws) cudaFree(h0->run_ws);
+        h0->run_ws = nullptr;
+        h0->device_bytes -= (size_t)h0->run_cap * each;
+        h0->run_cap = 0;
+        int rc = mol_dmalloc(h0, &h0->run_ws, (size_t)n * each);
+        if (rc) return rc;
+        h0->run_cap = n;
+    }
+    fgm::MolScalars *const out =
+        reinterpret_cast<fgm::MolScalars *>((char *)h0->run_ws + (size_t)h0->run_cap * 2 * sizeof(fgm::MolDesc));
     if (n > 1) {   // twice in a row, so that any rotation is one piece
         std::vector<fgm::MolDesc> v(2 * (size_t)n);
         for (int i = 0; i < n; i++) v[i] = v[n + i] = sys[i]->desc;
-        CK(cudaMalloc(&tmp, v.size() * sizeof(fgm::MolDesc)));
-        CK(cudaMemcpyAsync(tmp, v.data(), v.size() * sizeof(fgm::MolDesc), cudaMemcpyHostToDevice, st));
-        descs = tmp;
-    }
-    std::vector<fgm::MolScalars> s0(n), s1(n);
-    for (int i = 0; i < n; i++) {
-        CK(cudaMemcpyAsync(&s0[i], sys[i]->sc, sizeof(fgm::MolScalars), cudaMemcpyDeviceToHost, st));
+        CK(cudaMemcpyAsync(h0->run_ws, v.data(), v.size() * sizeof(fgm::MolDesc), cudaMemcpyHostToDevice, st));
+        descs = reinterpret_cast<const fgm::MolDesc *>(h0->run_ws);
     }
     CK(cudaEventRecord(h0->ev0, st));
     int rc = FG_OK;
@@ -1664,21 +1683,25 @@ int mol_run(fg_molsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
             rc = mol_launch(h0, L, descs + r * slots % n, slots, st, quantum);
     }
     CK(cudaEventRecord(h0->ev1, st));
-    CK(cudaEventSynchronize(h0->ev1));
     for (int i = 0; i < n; i++) sys[i]->staged = false;
-    if (tmp) cudaFree(tmp);
-    if (rc) return rc;
+    if (rc) {
+        cudaStreamSynchronize(st);
+        return rc;
+    }
+    // the scalars of all systems in one copy
+    fgm::mol_gather_kernel<<<(n + 127) / 128, 128, 0, st>>>(descs, n, out);
+    CK(cudaGetLastError());
+    std::vector<fgm::MolScalars> s1(n);
+    CK(cudaMemcpyAsync(s1.data(), out, (size_t)n * sizeof(fgm::MolScalars), cudaMemcpyDeviceToHost, st));
+    CK(cudaStreamSynchronize(st));
     float ms = 0.0f;
     CK(cudaEventElapsedTime(&ms, h0->ev0, h0->ev1));
-    for (int i = 0; i < n; i++)
-        CK(cudaMemcpyAsync(&s1[i], sys[i]->sc, sizeof(fgm::MolScalars), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
     fg_sweep_stats tot{};
     int errs = 0;
     for (int i = 0; i < n; i++) {
         fg_sweep_stats x{};
         x.trials = s1[i].cursor;
-        x.accepted = s1[i].n_accepted - sys[i]->acc0;
+        x.accepted = s1[i].n_accepted - s1[i].acc0;
         x.energy_change = df_val(s1[i].u_hi, s1[i].u_lo);
         x.device_ms = ms;
         x.sweep_kernel_ms = ms;

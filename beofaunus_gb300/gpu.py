@@ -159,7 +159,11 @@ def lib(build_if_missing=True):
 
 
 def _p(a):
-    return None if a is None else a.ctypes.data_as(ctypes.c_void_p)
+    if a is None:
+        return None
+    p = ctypes.c_void_p(a.ctypes.data)   # as data_as does, in half its time
+    p._arr = a                           # the pointer keeps the array
+    return p
 
 
 class TuneReport(ctypes.Structure):
