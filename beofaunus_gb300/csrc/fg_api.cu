@@ -3,6 +3,7 @@
 // parallel tempering and the job server are in fg_batch.cu (same
 // translation unit). See include/faunus_gb300.h.
 #include <algorithm>
+#include <chrono>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -136,6 +137,10 @@ struct fg_system {
     int nc[3] = {0, 0, 0};
     int cap = 0;
     bool trial_pending = false;
+    int32_t trial_idx = 0;                       // the pending trial: particle, new position
+    int64_t trial_x[3] = {0, 0, 0};
+    uint32_t trial_call = 0;                     // plain trials so far
+    unsigned long long *trial_host = nullptr;    // pinned: dU of the last plain trial (trial_kernel)
     bool state_set = false;
     int cnt_accepted_host = 0;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -154,6 +159,7 @@ void free_all(fg_system *h) {
                     h->eb_ranges, h->cl_items, h->d_desc_cl, h->work64};
     for (void *p : ptrs)
         if (p) cudaFree(p);
+    if (h->trial_host) cudaFreeHost(h->trial_host);
     if (h->ev0) cudaEventDestroy(h->ev0);
     if (h->ev1) cudaEventDestroy(h->ev1);
     if (h->stream) cudaStreamDestroy(h->stream);
@@ -308,8 +314,8 @@ size_t sweep_smem(const fg_system *h, bool pos_smem) {
 }
 
 using SweepFn = void (*)(const SysDesc *, int64_t, const float2 *);
-using TrialFn = void (*)(const SysDesc *, const int64_t *, float2 *, const float2 *);
-using CommitFn = void (*)(const SysDesc *, const int64_t *, const float2 *, const float2 *);
+using TrialFn = void (*)(const SysDesc *, fg::TrialArgs, int64_t *, float2 *, volatile unsigned long long *);
+using CommitFn = void (*)(const SysDesc *, fg::TrialArgs, const int64_t *, const float2 *);
 
 // Ewald systems run the block-of-trials kernel (fg_ewald_block.cu) when its
 // shared memory fits; 512 threads per system.
@@ -342,6 +348,25 @@ CommitFn commit_fn(const fg_system *h) {
     if (h->model == FG_MODEL_EWALD_WCA)
         return h->use_cells ? fg::commit_kernel<fg::MODEL_EWALD, true> : fg::commit_kernel<fg::MODEL_EWALD, false>;
     return fg::commit_kernel<fg::MODEL_DHLJ, false>;
+}
+
+fg::TrialArgs trial_args(const fg_system *h) {
+    return {h->pos64, h->pos4, h->ptype, h->kvec, h->kpack, h->qfix, h->sc, h->sc_tab, h->N, h->K, h->trial_idx, h->trial_call,
+            {h->trial_x[0], h->trial_x[1], h->trial_x[2]}};
+}
+
+// CTAs of a plain trial: a power of two (one cluster, at most 8) that leaves
+// a thread two or fewer items (k-vectors, and partners: all of them, or
+// those of the 27 stencil cells).
+// A call of 16384 salt ions takes 37 us on one CTA and 20 on eight, of 16384
+// Ewald ions with cells 23.9 and 21.8 (four); with one item a thread instead
+// (four CTAs at 800 ions) 20.5 against 19.8.
+int trial_ctas(const fg_system *h) {
+    const int64_t cells = h->use_cells ? (int64_t)h->nc[0] * h->nc[1] * h->nc[2] : 1;
+    const int64_t items = h->K + (h->use_cells ? (27 * (int64_t)h->N + cells - 1) / cells : (int64_t)h->N);
+    int C = 1;
+    while (C < 8 && items > 2 * (int64_t)C * fg::kTrialThreads) C *= 2;
+    return C;
 }
 
 int set_smem_attr(const void *fn, size_t bytes) {
@@ -1524,20 +1549,48 @@ int fg_trial_du(fg_system *h, int32_t n_moved, const int32_t *idx, const double 
     if (idx[0] < 0 || idx[0] >= h->N) return fail(FG_ERR_INVALID, "particle index out of range");
     for (int a = 0; a < 3; a++)
         if (!std::isfinite(new_xyz[a])) return fail(FG_ERR_INVALID, "non-finite coordinate");
-    const int64_t req[4] = {idx[0], to_fix(new_xyz[0], h->P.box[0]), to_fix(new_xyz[1], h->P.box[1]),
-                            to_fix(new_xyz[2], h->P.box[2])};
-    CK(cudaMemcpyAsync(h->req, req, sizeof(req), cudaMemcpyHostToDevice, h->stream));
-    const int T = sweep_threads(h);
-    const size_t sm = sweep_smem(h, false);
-    TrialFn fn = trial_fn(h);
-    int rc = set_smem_attr((const void *)fn, sm);
-    if (rc) return rc;
-    fn<<<1, T, sm, h->stream>>>(h->d_desc, h->req, h->trial_out, h->sc_tab);
-    CK(cudaGetLastError());
-    float2 out[3];
-    CK(cudaMemcpyAsync(out, h->trial_out, sizeof(out), cudaMemcpyDeviceToHost, h->stream));
-    CK(cudaStreamSynchronize(h->stream));
-    *du = df_val(out[0].x, out[0].y);
+    if (sweep_smem(h, false) + sizeof(SysDesc) > 227 * 1024)   // as for a sweep
+        return fail(FG_ERR_CUDA, "%d k-vectors do not fit in shared memory", h->K);
+    if (!h->trial_host) {
+        CK(cudaHostAlloc((void **)&h->trial_host, 2 * sizeof(*h->trial_host), cudaHostAllocMapped | cudaHostAllocPortable));
+        h->trial_host[0] = h->trial_host[1] = 0;
+    }
+    h->trial_idx = idx[0];
+    for (int x = 0; x < 3; x++) h->trial_x[x] = to_fix(new_xyz[x], h->P.box[x]);
+    h->trial_call++;
+    const fg::TrialArgs a = trial_args(h);
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)trial_ctas(h);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.gridDim = dim3(attr[0].val.clusterDim.x);
+    cfg.blockDim = dim3(fg::kTrialThreads);
+    cfg.stream = h->stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = cfg.gridDim.x > 1 ? 1 : 0;
+    CK(cudaLaunchKernelEx(&cfg, trial_fn(h), (const SysDesc *)h->d_desc, a, h->req, h->trial_out,
+                          (volatile unsigned long long *)h->trial_host));
+    // dU arrives in pinned memory; a synchronisation (and its error, if any)
+    // only if it has not within a few milliseconds
+    unsigned long long w[2];
+    bool synced = false;
+    const auto t0 = std::chrono::steady_clock::now();
+    for (unsigned spin = 0;; spin++) {
+        for (int x = 0; x < 2; x++) w[x] = __atomic_load_n(&h->trial_host[x], __ATOMIC_ACQUIRE);
+        if ((uint32_t)(w[0] >> 32) == a.call && (uint32_t)(w[1] >> 32) == a.call) break;
+        if (synced) return fail(FG_ERR_DEVICE, "the trial's result did not arrive");
+        if ((spin & 1023) == 1023 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
+            CK(cudaStreamSynchronize(h->stream));
+            synced = true;
+        }
+    }
+    float out[2];
+    for (int x = 0; x < 2; x++) {
+        const uint32_t bits = (uint32_t)w[x];
+        std::memcpy(&out[x], &bits, 4);
+    }
+    *du = df_val(out[0], out[1]);
     h->trial_pending = true;
     return FG_OK;
 }
@@ -1548,12 +1601,9 @@ int fg_commit(fg_system *h, int32_t accepted, double *correction) {
     h->trial_pending = false;
     if (correction) *correction = 0.0;
     if (!accepted) return FG_OK;
-    const int T = sweep_threads(h);
-    const size_t sm = sweep_smem(h, false);
-    CommitFn fn = commit_fn(h);
-    int rc = set_smem_attr((const void *)fn, sm);
-    if (rc) return rc;
-    fn<<<1, T, sm, h->stream>>>(h->d_desc, h->req, h->trial_out, h->sc_tab);
+    const int grid = std::max(1, (h->K + fg::kTrialThreads - 1) / fg::kTrialThreads);
+    const size_t sm = 2 * (size_t)fg::qk_tab_len(h->kc) * sizeof(float2);   // axis tables
+    commit_fn(h)<<<grid, fg::kTrialThreads, sm, h->stream>>>(h->d_desc, trial_args(h), h->req, h->trial_out);
     CK(cudaGetLastError());
     if (h->model == FG_MODEL_EWALD_WCA && !h->desc.skip_rebuild) {
         // the host mirrors the rebuild counter (NonbondedEwald::update, ewald.h:633)
@@ -1561,7 +1611,7 @@ int fg_commit(fg_system *h, int32_t accepted, double *correction) {
             h->cnt_accepted_host = 0;
             const int one = 1;
             CK(cudaMemcpyAsync(&h->sc->rebuild_pending, &one, sizeof(int), cudaMemcpyHostToDevice, h->stream));
-            rc = launch_rebuild(h->d_desc, 1, h->N, h->nseg, h->kc, h->corr, h->stream);
+            int rc = launch_rebuild(h->d_desc, 1, h->N, h->nseg, h->kc, h->corr, h->stream);
             if (rc) return rc;
             float2 e;
             CK(cudaMemcpyAsync(&e, h->corr, sizeof(e), cudaMemcpyDeviceToHost, h->stream));

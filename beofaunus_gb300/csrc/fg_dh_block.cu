@@ -34,25 +34,6 @@ namespace fg {
 constexpr int kBlkTrials = 32;
 constexpr int kBlkThreads = 512;
 
-__device__ __forceinline__ unsigned blk_cluster_rank() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ unsigned blk_cluster_size() {
-    unsigned r;
-    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-    return r;
-}
-__device__ __forceinline__ void blk_cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ void blk_st_cluster(float2 *p, unsigned rank, float2 v) {
-    unsigned a = (unsigned)__cvta_generic_to_shared(p), ra;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(rank));
-    asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(ra), "f"(v.x), "f"(v.y) : "memory");
-}
-
 struct __align__(16) BlkView {   // one trial
     int hx, hy, hz;        // old high words
     float dx, dy, dz, d2;  // step (words), its square
