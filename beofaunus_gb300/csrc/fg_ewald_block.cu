@@ -741,6 +741,32 @@ __device__ __forceinline__ void cq_pass(const float4 *tab, int T, const float *q
         }
     }
 }
+// Adds an item's differences to its k-vectors' Q(k).
+__device__ __forceinline__ void eb_commit_item(const EbSmem &s, int kp0, int kn0, int n0, int len, int shift,
+                                               const unsigned da[kRbLen], const unsigned dr[kRbLen],
+                                               const unsigned db[kRbLen], const unsigned dc[kRbLen]) {
+#pragma unroll
+    for (int u = 0; u < kRbLen; u++) {
+        if (u >= len) continue;
+        // +n: (a - r, b + c); -n: (a + r, c - b)
+        longlong2 q = s.b.qfix[kp0 + u];
+        q.x += qk_widen((int)(da[u] - dr[u]), shift);
+        q.y += qk_widen((int)(db[u] + dc[u]), shift);
+        s.b.qfix[kp0 + u] = q;
+        float2 qf = q_to_float(q);
+        s.b.kvec[kp0 + u].y = qf.x;
+        s.b.kvec[kp0 + u].z = qf.y;
+        if (n0 + u > 0) {
+            q = s.b.qfix[kn0 - u];
+            q.x += qk_widen((int)(da[u] + dr[u]), shift);
+            q.y += qk_widen((int)(dc[u] - db[u]), shift);
+            s.b.qfix[kn0 - u] = q;
+            qf = q_to_float(q);
+            s.b.kvec[kn0 - u].y = qf.x;
+            s.b.kvec[kn0 - u].z = qf.y;
+        }
+    }
+}
 // Q(k) after a block: every accepted trial a adds c_k(new_a) - c_k(old_a)
 // (ewald.h:665-705). Threads qt = 0..nq-1 (warps 1.. of the CTA, which
 // synchronise among themselves on named barrier 1) own the rebuild's items
@@ -793,27 +819,7 @@ __device__ __noinline__ void eb_commit_qk(const SysDesc &d, const EbSmem &s, uin
                 case 3: cq_pass<3>(tab, T, qg + g0, ng, ix, iy, iz, da, dr, db, dc); break;
                 default: cq_pass<4>(tab, T, qg + g0, ng, ix, iy, iz, da, dr, db, dc); break;
             }
-#pragma unroll
-            for (int u = 0; u < kRbLen; u++) {
-                if (u >= len) continue;
-                // +n: (a - r, b + c); -n: (a + r, c - b)
-                longlong2 q = s.b.qfix[kp0 + u];
-                q.x += qk_widen((int)(da[u] - dr[u]), shift);
-                q.y += qk_widen((int)(db[u] + dc[u]), shift);
-                s.b.qfix[kp0 + u] = q;
-                float2 qf = q_to_float(q);
-                s.b.kvec[kp0 + u].y = qf.x;
-                s.b.kvec[kp0 + u].z = qf.y;
-                if (n0 + u > 0) {
-                    q = s.b.qfix[kn0 - u];
-                    q.x += qk_widen((int)(da[u] + dr[u]), shift);
-                    q.y += qk_widen((int)(dc[u] - db[u]), shift);
-                    s.b.qfix[kn0 - u] = q;
-                    qf = q_to_float(q);
-                    s.b.kvec[kn0 - u].y = qf.x;
-                    s.b.kvec[kn0 - u].z = qf.y;
-                }
-            }
+            eb_commit_item(s, kp0, kn0, n0, len, shift, da, dr, db, dc);
         }
     }
 }
@@ -1205,7 +1211,9 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
             if (rank == 0) {
                 for (int e = tid; e < kEbGramN; e += blockDim.x) {
                     float v = 0.0f;
-                    for (int r = 0; r < C; r++) v += s.xgram[r * kEbGramN + e];
+#pragma unroll
+                    for (int r = 0; r < kEbMaxCluster; r++)   // all loads in flight at once
+                        if (r < C) v += s.xgram[r * kEbGramN + e];
                     const int x = e >> 7, ln = (e >> 2) & 31, j = e & 3;
                     const int mi = x < 4 ? 0 : 1, nj = x < 4 ? x : x - 2;
                     const int row = 16 * mi + (ln >> 2) + ((j & 2) ? 8 : 0);
@@ -1248,33 +1256,35 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
             // NonbondedEwald::update (ewald.h:633): a rebuild after
             // update_frequency accepted trials ends the block there
             const int every = max(uf, 1), left = d.skip_rebuild ? 64 : max(every - cnt_acc, 1);
-            const bool due = left <= kb;   // a rebuild may fall due in this block
+            // Lane a decides: its S already holds the corrections of every
+            // accepted trial before it in the block. Movebase::metropolis
+            // (move.h:567-573): reject iff dU > kT (-ln u); a NaN dU compares
+            // false there: accepted. Every lane forms its flag and the sum it
+            // would go on with; bit a of the flags' ballot selects. A step is
+            // that chain alone, without a branch (180 -> 85 cycles): where the
+            // block ends is found afterwards, the sums of the trials before that
+            // not depending on the later ones.
             float2 cn = s.corr[lane];
+#pragma unroll 4
             for (int a = 0; a < kb; a++) {
-                // lane a decides: its S already holds the corrections of every
-                // accepted trial before it in the block. Movebase::metropolis
-                // (move.h:567-573): reject iff dU > kT (-ln u); a NaN dU
-                // compares false there: accepted. Every lane forms its flags and
-                // the sum it would go on with; bit a of their ballots selects, so
-                // a step has no divergent branch
                 const float2 c = cn;
                 cn = s.corr[min(a + 1, kEbTrials - 1) * kEbTrials + lane];
                 const df Sc = df_add_quick(S, df{c.x, c.y});
-                const uint32_t again = __ballot_sync(0xffffffffu, (colm & accm) != 0u);
-                const uint32_t ok = __ballot_sync(0xffffffffu, !df_gt(S, df{th.x, th.y}));
-                if ((again >> a) & 1u) {   // its particle was moved by an accepted trial of this block
-                    done = a;
-                    break;
-                }
-                accm |= ok & (1u << a);
-                const bool add = ((ok >> a) & 1u) && lane > a;
+                const bool gt = S.hi > th.x || (S.hi == th.x && S.lo > th.y);
+                const uint32_t ok = __ballot_sync(0xffffffffu, !gt) & (1u << a);
+                accm |= ok;
+                const bool add = ok && lane > a;
                 S.hi = add ? Sc.hi : S.hi;
                 S.lo = add ? Sc.lo : S.lo;
-                if (due && __popc(accm) == left) {
-                    rebuild = true;
-                    done = a + 1;
-                    break;
-                }
+            }
+            // a trial whose particle an accepted one moved ends the block
+            const uint32_t again = __ballot_sync(0xffffffffu, (colm & accm) != 0u);
+            if (again) done = __ffs(again) - 1;
+            if (done < 32) accm &= (1u << done) - 1u;
+            if (__popc(accm) >= left) {   // and so does the accepted one that makes a rebuild due
+                rebuild = true;
+                done = (int)__fns(accm, 0, left) + 1;
+                if (done < 32) accm &= (1u << done) - 1u;
             }
             nacc += __popc(accm);
             cnt_acc = rebuild ? 0 : (cnt_acc + __popc(accm)) % every;
