@@ -69,7 +69,7 @@ struct DipTrial {
 
 struct DipScalars {
     int64_t cursor;       // next trial of the staged stream
-    int64_t acc0;         // n_accepted when the stream was staged
+    int64_t n_trials;     // end of the stream for this launch
     int64_t n_accepted;   // cumulative
     int64_t n_rebuilds;   // cumulative Q(k) rebuilds
     int32_t error;
@@ -80,6 +80,7 @@ struct DipScalars {
     double drift;         // NonbondedEwald::update_drift
     double pend_du;       // dU of an evaluated explicit trial
     double M[6];          // surface sums: sum q eff r (3), sum mu_s mu (3)
+    int64_t acc0;         // n_accepted when the stream was staged
 };
 
 struct DipDesc {
@@ -542,38 +543,44 @@ __global__ void __launch_bounds__(kDipMaxThreads, 1) dip_build_kernel(const DipD
     dip_rebuild(d, A, S, before, after);
 }
 
-// mode 0: run the staged stream [cursor, end) with Metropolis decisions;
+// mode 0: run the staged stream [cursor, n_trials) with Metropolis decisions;
 // mode 1: evaluate trials[0] (explicit) and keep it pending;
 // mode 2: apply the pending trials[0] as accepted.
 // MAXT: the launch bound. 128 threads per system at most 128 registers
 // (four systems, sixteen warps on an SM) or up to kDipMaxThreads at one CTA
 // per SM.
-// The systems of a launch: one, or many by their device descriptors with the
-// ends of their streams (no trial of index cap or above runs).
-struct DipLaunch {
-    const DipDesc *one;
-    const DipDesc *const *many;
-    const int64_t *ends;
-    int64_t end, cap;
-};
-
 // A newly staged stream: cursor, per-stream sum and flags from zero.
 __global__ void dip_begin_kernel(DipScalars *sc) {
     sc->cursor = 0;
+    sc->n_trials = 0;
     sc->acc0 = sc->n_accepted;
     sc->usum = 0.0;
     sc->error = 0;
 }
-// The scalars of many systems into one array (one copy to the host).
-__global__ void dip_gather_kernel(DipLaunch l, int n, DipScalars *out) {
+// The descriptors of many systems side by side (the sweep kernel takes them as
+// one read-only array: reached through a pointer loaded per block, their
+// fields were loaded again and again, 9 % of a single system's sweep).
+__global__ void dip_descs_kernel(const DipDesc *const *from, DipDesc *to) {
+    const int32_t *a = reinterpret_cast<const int32_t *>(from[blockIdx.x]);
+    int32_t *b = reinterpret_cast<int32_t *>(to + blockIdx.x);
+    for (int t = threadIdx.x; t < (int)(sizeof(DipDesc) / 4); t += blockDim.x) b[t] = a[t];
+}
+// The next launch's ends: each system's stream (ends; end for one system) up
+// to trial cap.
+__global__ void dip_ends_kernel(const DipDesc *descs, int n, const int64_t *ends, int64_t end, int64_t cap) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = l.many ? *l.many[i]->sc : *l.one->sc;
+    if (i < n) descs[i].sc->n_trials = min(ends ? ends[i] : end, cap);
+}
+// The scalars of many systems into one array (one copy to the host).
+__global__ void dip_gather_kernel(const DipDesc *descs, int n, DipScalars *out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = *descs[i].sc;
 }
 
 template <int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(DipLaunch l, int mode, int stage) {
-    const DipDesc *__restrict__ dp = l.many ? l.many[blockIdx.x] : l.one;
-    const DipDesc &d = *dp;
+__global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(const DipDesc *__restrict__ descs, int mode,
+                                                                               int stage) {
+    const DipDesc &d = descs[blockIdx.x];
     __shared__ DipShared S;
     extern __shared__ __align__(16) unsigned char dsm[];
     float4 *eyz = reinterpret_cast<float4 *>(dsm);   // df complex
@@ -623,7 +630,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(Di
     int64_t t0 = 0, t1 = 1;
     if (mode == 0) {
         t0 = d.sc->cursor;
-        t1 = min(l.many ? l.ends[blockIdx.x] : l.end, l.cap);
+        t1 = d.sc->n_trials;
     }
     DipTrial nxt;   // lanes 0..2: the next trial's record, loaded one trial ahead
     if (tid < 3 && t0 < t1) nxt = d.trials[mode == 0 ? t0 : 0];
@@ -938,6 +945,9 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(Di
     if (tid == 0) {
         if (mode == 0) sc.cursor = t1;
         for (int a = 0; a < 6; a++) sc.M[a] = S.M[a];
+        // not held in registers over the launch
+        sc.n_trials = d.sc->n_trials;
+        sc.acc0 = d.sc->acc0;
         *d.sc = sc;
     }
 }
@@ -996,8 +1006,8 @@ struct fg_dipsys {
     int64_t log_cap = 0;
     fgd::DipScalars *sc = nullptr;
     int64_t n_stream = 0;
-    // dip_run's workspace of the system it launches from: n descriptor
-    // pointers, n stream ends, n scalars
+    // dip_run's workspace of the system it launches from: n descriptors, n
+    // pointers to them, n stream ends, n scalars
     void *run_ws = nullptr;
     int run_cap = 0;
     fgd::DipDesc pushed{};   // what d_desc holds
@@ -1330,7 +1340,7 @@ size_t dip_launch_smem(fg_dipsys *const *sys, int n, int &stage) {
     return stage ? st : yz;
 }
 
-int dip_launch(fg_dipsys *const *sys, const fgd::DipLaunch &l, int n, int mode, cudaStream_t st) {
+int dip_launch(fg_dipsys *const *sys, const fgd::DipDesc *descs, int n, int mode, cudaStream_t st) {
     int stage = 0;
     size_t smem = dip_launch_smem(sys, n, stage);
     if (mode != 0) {
@@ -1341,9 +1351,9 @@ int dip_launch(fg_dipsys *const *sys, const fgd::DipLaunch &l, int n, int mode, 
     const void *fn = T <= 128 ? (const void *)fgd::dip_sweep_kernel<128> : (const void *)fgd::dip_sweep_kernel<fgd::kDipMaxThreads>;
     CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     if (T <= 128)
-        fgd::dip_sweep_kernel<128><<<n, T, smem, st>>>(l, mode, stage);
+        fgd::dip_sweep_kernel<128><<<n, T, smem, st>>>(descs, mode, stage);
     else
-        fgd::dip_sweep_kernel<fgd::kDipMaxThreads><<<n, T, smem, st>>>(l, mode, stage);
+        fgd::dip_sweep_kernel<fgd::kDipMaxThreads><<<n, T, smem, st>>>(descs, mode, stage);
     CK(cudaGetLastError());
     return FG_OK;
 }
@@ -1366,7 +1376,7 @@ int dip_run(fg_dipsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
     // (8 bytes in and 136 out for each of 608 systems, one at a time, and
     // their descriptors were 8 ms beside an 18 ms kernel).
     if (h0->run_cap < n) {
-        const size_t each = sizeof(void *) + sizeof(int64_t) + sizeof(fgd::DipScalars);
+        const size_t each = sizeof(fgd::DipDesc) + sizeof(void *) + sizeof(int64_t) + sizeof(fgd::DipScalars);
         if (h0->run_ws) cudaFree(h0->run_ws);
         h0->run_ws = nullptr;
         h0->device_bytes -= (size_t)h0->run_cap * each;
@@ -1375,17 +1385,24 @@ int dip_run(fg_dipsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
         if (rc) return rc;
         h0->run_cap = n;
     }
-    fgd::DipScalars *const out = reinterpret_cast<fgd::DipScalars *>((char *)h0->run_ws + (size_t)16 * h0->run_cap);
-    fgd::DipLaunch l{h0->d_desc, nullptr, nullptr, h0->n_stream, 0};
+    static_assert(sizeof(fgd::DipDesc) % 8 == 0 && sizeof(fgd::DipScalars) % 8 == 0, "run_ws");
+    fgd::DipDesc *const all = (fgd::DipDesc *)h0->run_ws;
+    int64_t *const in = reinterpret_cast<int64_t *>(all + h0->run_cap);
+    fgd::DipScalars *const out = reinterpret_cast<fgd::DipScalars *>(in + 2 * (size_t)h0->run_cap);
+    const fgd::DipDesc *descs = h0->d_desc;
+    const int64_t *ends = nullptr;
+    const int64_t end = h0->n_stream;
     if (n > 1) {
         std::vector<int64_t> v(2 * (size_t)n);
         for (int i = 0; i < n; i++) {
             v[i] = (int64_t)(intptr_t)sys[i]->d_desc;
             v[n + i] = sys[i]->n_stream;
         }
-        CK(cudaMemcpyAsync(h0->run_ws, v.data(), v.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
-        l.many = reinterpret_cast<const fgd::DipDesc *const *>(h0->run_ws);
-        l.ends = reinterpret_cast<const int64_t *>(h0->run_ws) + n;
+        CK(cudaMemcpyAsync(in, v.data(), v.size() * sizeof(int64_t), cudaMemcpyHostToDevice, st));
+        fgd::dip_descs_kernel<<<n, 128, 0, st>>>(reinterpret_cast<const fgd::DipDesc *const *>(in), all);
+        CK(cudaGetLastError());
+        descs = all;
+        ends = in + n;
     }
     // launches of at most kChunk trials per system keep each kernel short
     const int64_t kChunk = 16384;
@@ -1393,15 +1410,16 @@ int dip_run(fg_dipsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
     CK(cudaEventRecord(h0->ev0, st));
     int rc = FG_OK;
     for (int64_t c = 0; c < nl && !rc; c++) {
-        l.cap = (c + 1) * kChunk;
-        rc = dip_launch(sys, l, n, 0, st);
+        fgd::dip_ends_kernel<<<(n + 127) / 128, 128, 0, st>>>(descs, n, ends, end, (c + 1) * kChunk);
+        CK(cudaGetLastError());
+        rc = dip_launch(sys, descs, n, 0, st);
     }
     CK(cudaEventRecord(h0->ev1, st));
     if (rc) {
         cudaStreamSynchronize(st);
         return rc;
     }
-    fgd::dip_gather_kernel<<<(n + 127) / 128, 128, 0, st>>>(l, n, out);
+    fgd::dip_gather_kernel<<<(n + 127) / 128, 128, 0, st>>>(descs, n, out);
     CK(cudaGetLastError());
     std::vector<fgd::DipScalars> s1(n);
     CK(cudaMemcpyAsync(s1.data(), out, (size_t)n * sizeof(fgd::DipScalars), cudaMemcpyDeviceToHost, st));
@@ -1793,7 +1811,7 @@ int fg_dip_trial_du(fg_dipsys *h, int32_t i, const double *new_xyz, const double
     int rc = dip_ensure_trials(h, 1, false);
     if (rc) return rc;
     CK(cudaMemcpyAsync(h->trials, &t, sizeof(t), cudaMemcpyHostToDevice, h->stream));
-    rc = dip_launch(&h, {h->d_desc, nullptr, nullptr, 0, 0}, 1, 1, h->stream);
+    rc = dip_launch(&h, h->d_desc, 1, 1, h->stream);
     if (rc) return rc;
     fgd::DipScalars s;
     rc = dip_read_scalars(h, s);
@@ -1812,7 +1830,7 @@ int fg_dip_commit(fg_dipsys *h, int32_t accepted, double *correction) {
     if (!accepted) return FG_OK;
     fgd::DipScalars s0, s1;
     int rc = dip_read_scalars(h, s0);
-    if (!rc) rc = dip_launch(&h, {h->d_desc, nullptr, nullptr, 0, 0}, 1, 2, h->stream);
+    if (!rc) rc = dip_launch(&h, h->d_desc, 1, 2, h->stream);
     if (!rc) rc = dip_read_scalars(h, s1);
     if (rc) return rc;
     // what update() returns: the reciprocal-energy change of a Q(k) rebuild
