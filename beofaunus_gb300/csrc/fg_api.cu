@@ -435,12 +435,14 @@ int eb_cluster_max(fg_system *h) {
 }
 
 // CTAs of the cluster a system alone runs on: the requested size, or the
-// built-in choice (as many as fit, with no fewer than 128 k-vectors per CTA;
-// 16 on 16384 ions with K = 2242 runs 0.89 us per trial against 1.03 on 8
-// and 3.23 on one), capped by what fits.
+// built-in choice (as many as fit, with no fewer than 32 k-vectors per CTA),
+// capped by what fits. Microseconds per trial on 1, 4, 8 and 16 CTAs: 16384
+// ions, K = 2242 2.48, 1.07, 0.84, 0.74; 800 ions, K = 783 1.42, 0.82, 0.68,
+// 0.64; 800 ions, K = 297 1.11, 0.74, 0.65, 0.63; 100 ions, K = 297 1.63, 1.27,
+// 1.20, 1.26.
 int eb_cluster_ctas(fg_system *h) {
     if (h->model != FG_MODEL_EWALD_WCA || h->K <= 0 || !ewald_block_ok(h)) return 1;
-    const int want = h->eb_ctas > 0 ? h->eb_ctas : std::max(1, std::min(fg::kEbMaxCluster, h->K / 128));
+    const int want = h->eb_ctas > 0 ? h->eb_ctas : std::max(1, std::min(fg::kEbMaxCluster, h->K / 32));
     const int maxc = eb_cluster_max(h);
     int C = 1;
     while (2 * C <= std::min(want, maxc)) C *= 2;
