@@ -103,7 +103,8 @@ struct fg_system {
     longlong2 *qfix = nullptr, *qnew = nullptr;
     SysScalars *sc = nullptr;
     float2 *trial_out = nullptr, *corr = nullptr, *pair_part = nullptr;
-    int64_t *req = nullptr, *dp_fix = nullptr;
+    unsigned *ticket = nullptr;    // commit_kernel's (zero between launches)
+    int64_t *dp_fix = nullptr;
     float2 *sc_tab = nullptr;
     Trial *trials = nullptr;
     int64_t trials_cap = 0, n_trials = 0;
@@ -154,7 +155,7 @@ namespace {
 void free_all(fg_system *h) {
     void *ptrs[] = {h->d_desc, h->pos64, h->pos4, h->pos_ext, h->cell_ext, h->ptype, h->cell_count, h->cell_pid,
                     h->p_cell, h->p_slot, h->cell_pos, h->kvec, h->core_tab, h->core_tab2, h->kpack, h->qfix,
-                    h->qnew, h->sc, h->trial_out, h->corr, h->pair_part, h->req, h->dp_fix, h->sc_tab, h->trials,
+                    h->qnew, h->sc, h->trial_out, h->corr, h->pair_part, h->ticket, h->dp_fix, h->sc_tab, h->trials,
                     h->log_du, h->log_acc, h->kseg, h->rb_items, h->raw_idx, h->raw_disp, h->raw_u,
                     h->eb_ranges, h->cl_items, h->d_desc_cl, h->work64};
     for (void *p : ptrs)
@@ -314,8 +315,8 @@ size_t sweep_smem(const fg_system *h, bool pos_smem) {
 }
 
 using SweepFn = void (*)(const SysDesc *, int64_t, const float2 *);
-using TrialFn = void (*)(const SysDesc *, fg::TrialArgs, int64_t *, float2 *, volatile unsigned long long *);
-using CommitFn = void (*)(const SysDesc *, fg::TrialArgs, const int64_t *, const float2 *);
+using TrialFn = void (*)(const SysDesc *, fg::TrialArgs, float2 *, volatile unsigned long long *);
+using CommitFn = void (*)(const SysDesc *, fg::TrialArgs, unsigned *, const float2 *);
 
 // Ewald systems run the block-of-trials kernel (fg_ewald_block.cu) when its
 // shared memory fits; 512 threads per system.
@@ -1228,7 +1229,8 @@ int fg_create(const fg_params *params, int32_t n_particles, fg_system **out) {
     ALLOC(h->pos_ext, (size_t)N * sizeof(short4));
     ALLOC(h->ptype, (size_t)N);
     ALLOC(h->sc, sizeof(SysScalars));
-    ALLOC(h->req, 8 * sizeof(int64_t));
+    ALLOC(h->ticket, sizeof(unsigned));
+    if (cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), h->stream) != cudaSuccess) return bail(fail(FG_ERR_CUDA, "ticket"));
     ALLOC(h->trial_out, 4 * sizeof(float2));
     ALLOC(h->corr, 4 * sizeof(float2));
     ALLOC(h->sc_tab, 256 * sizeof(float2));
@@ -1571,7 +1573,7 @@ int fg_trial_du(fg_system *h, int32_t n_moved, const int32_t *idx, const double 
     cfg.stream = h->stream;
     cfg.attrs = attr;
     cfg.numAttrs = cfg.gridDim.x > 1 ? 1 : 0;
-    CK(cudaLaunchKernelEx(&cfg, trial_fn(h), (const SysDesc *)h->d_desc, a, h->req, h->trial_out,
+    CK(cudaLaunchKernelEx(&cfg, trial_fn(h), (const SysDesc *)h->d_desc, a, h->trial_out,
                           (volatile unsigned long long *)h->trial_host));
     // dU arrives in pinned memory; a synchronisation (and its error, if any)
     // only if it has not within a few milliseconds
@@ -1605,7 +1607,7 @@ int fg_commit(fg_system *h, int32_t accepted, double *correction) {
     if (!accepted) return FG_OK;
     const int grid = std::max(1, (h->K + fg::kTrialThreads - 1) / fg::kTrialThreads);
     const size_t sm = 2 * (size_t)fg::qk_tab_len(h->kc) * sizeof(float2);   // axis tables
-    commit_fn(h)<<<grid, fg::kTrialThreads, sm, h->stream>>>(h->d_desc, trial_args(h), h->req, h->trial_out);
+    commit_fn(h)<<<grid, fg::kTrialThreads, sm, h->stream>>>(h->d_desc, trial_args(h), h->ticket, h->trial_out);
     CK(cudaGetLastError());
     if (h->model == FG_MODEL_EWALD_WCA && !h->desc.skip_rebuild) {
         // the host mirrors the rebuild counter (NonbondedEwald::update, ewald.h:633)

@@ -931,7 +931,7 @@ struct TrialArgs {
 };
 template <int MODEL, bool CELLS>
 __global__ void __launch_bounds__(kTrialThreads) trial_kernel(const SysDesc *__restrict__ dsc, TrialArgs a,
-                                                              int64_t *__restrict__ old, float2 *__restrict__ out,
+                                                              float2 *__restrict__ out,
                                                               volatile unsigned long long *host) {
     __shared__ __align__(16) SysDesc sd;
     __shared__ float2 tab[256], red[kTrialThreads / 32], part[8];
@@ -1021,7 +1021,6 @@ __global__ void __launch_bounds__(kTrialThreads) trial_kernel(const SysDesc *__r
         out[0] = make_float2(du.hi, du.lo);
         out[1] = make_float2(dM[0], dM[1]);
         out[2] = make_float2(dM[2], 0.0f);
-        for (int x = 0; x < 3; x++) old[x] = xo[x];
     }
 }
 
@@ -1066,14 +1065,17 @@ __device__ __forceinline__ void commit_position_global(const Move &m, const SysD
     d.p_slot[m.i] = ns;
 }
 
-// Movebase acceptMove + NonbondedEwald::update for the last plain trial. Its
-// old position comes from the trial (old), so no CTA reads what another
-// writes: the k-vectors spread over the grid, the last warp of CTA 0 commits the
-// position and the sums meanwhile. 4.7 -> 3.1 us at 783 k-vectors, against
-// staging k-vectors and cell tables in shared memory and storing them back.
+// Movebase acceptMove + NonbondedEwald::update for the last plain trial. The
+// particle's old position is the one it has now: a batch run between the trial
+// and its commit may have moved it, and Q(k) and the cell lists must lose the
+// position that they hold. The k-vectors spread over the grid, and every CTA
+// reads that position; so the last warp of the CTA that is last to have read it
+// (ticket, left at zero) commits the new one and the sums, while the others
+// update Q(k). 4.7 -> 3.1 us at 783 k-vectors, against staging k-vectors and
+// cell tables in shared memory and storing them back.
 template <int MODEL, bool CELLS>
 __global__ void __launch_bounds__(kTrialThreads) commit_kernel(const SysDesc *__restrict__ dsc, TrialArgs a,
-                                                               const int64_t *__restrict__ old,
+                                                               unsigned *__restrict__ ticket,
                                                                const float2 *__restrict__ trial_out) {
     extern __shared__ __align__(16) char smem_raw[];   // axis tables
     __shared__ __align__(16) SysDesc sd;
@@ -1083,7 +1085,7 @@ __global__ void __launch_bounds__(kTrialThreads) commit_kernel(const SysDesc *__
     int64_t xo[3], xn[3];
 #pragma unroll
     for (int x = 0; x < 3; x++) {
-        xo[x] = old[x];
+        xo[x] = a.pos64[3 * a.idx + x];
         xn[x] = a.x[x];
     }
     const float q = __int_as_float(a.pos4[a.idx].w);
@@ -1095,11 +1097,17 @@ __global__ void __launch_bounds__(kTrialThreads) commit_kernel(const SysDesc *__
         qk = a.qfix[g];
     }
     for (int t = tid; t < 256; t += T) tab[t] = a.sc_tab[t];
-    load_desc(sd, dsc);   // synchronises
+    load_desc(sd, dsc);   // synchronises: every thread of the CTA has read the old position
     const SysDesc &d = sd;
     Move m;
     move_setup(m, a.idx, xo, xn, q, ti, d);
-    if (g == T - 1) {
+    bool last = tid == T - 1;
+    if (last && gridDim.x > 1) {
+        __threadfence();
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+        if (last) *ticket = 0u;
+    }
+    if (last) {
         commit_position_global(m, d, CELLS);
         SysScalars *sc = d.sc;
         const df du = {trial_out[0].x, trial_out[0].y};

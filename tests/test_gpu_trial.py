@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from beofaunus_gb300 import workloads
-from beofaunus_gb300.gpu import System
+from beofaunus_gb300.gpu import Batch, System
 from oracle.oracle import OracleSystem
 
 pytestmark = pytest.mark.gpu
@@ -52,3 +52,38 @@ def test_trials_and_commits(name):
     assert np.abs(d - L * np.round(d / L)).max() < 1e-9
     if not name.startswith("salt"):
         assert s.rebuild_qk() == 0.0   # exact: the rebuild finds what the commits kept
+
+
+@pytest.mark.parametrize("name", ["rpm 240", "rpm 3000 cells", "salt 1030"])
+def test_commit_after_a_batch_run_moved_the_particle(name):
+    """The commit takes the particle from where it is, not from where it was
+    when the trial was evaluated: positions, exact Q(k) and cell lists hold."""
+    data = CASES[name]()
+    s, o = System(*data), OracleSystem(*data)
+    L, n = data[0].box[0], len(data[1])
+    rng = np.random.default_rng(n + 1)
+    i = n // 2
+    idx = rng.integers(0, n, 200).astype(np.int32)
+    idx[::4] = i
+    disp = 2.0 * (rng.random((200, 3)) - 0.5)
+    disp[::4, 0] = 2.5                      # through several cells
+    st = (idx, disp, np.full(200, 1e-3))
+    batch = Batch([s])
+    batch.stream_upload(0, *st)
+    new = s.positions()[i] + 0.3
+    new -= L * np.floor(new / L + 0.5)
+    s.trial_du(i, new)
+    batch.run()
+    s.commit(True)
+    o.mc_run_stream(*st)
+    o.trial_du(i, new)
+    o.commit(True)
+    d = s.positions() - o.positions()
+    assert np.abs(d - L * np.round(d / L)).max() < 1e-9
+    if not name.startswith("salt"):
+        assert s.rebuild_qk() == 0.0
+    st = (rng.integers(0, n, 300).astype(np.int32), 2.0 * (rng.random((300, 3)) - 0.5), rng.random(300))
+    r, ro = s.sweep(*st), o.mc_run_stream(*st)
+    np.testing.assert_array_equal(r["acc"], ro["acc"])
+    # up to 60 near terms of 2 kT, three FP32 roundings each (3e-6), and the reciprocal sum (1e-6)
+    assert np.all(np.abs(r["du"] - ro["du"]) < 5e-6 + 1e-9 * np.abs(ro["du"]))
