@@ -251,6 +251,21 @@ __device__ __forceinline__ void move_setup(Move &m, int i, const int64_t xo[3], 
     }
 }
 
+// r_n^2 - r_o^2 of pair (p, moved particle) in squared high-word units, exact in
+// integers: sum_a (dn_a - do_a)(dn_a + do_a), each minimum image taken
+// separately. A term is below 2^62, three of them (a step through much of the
+// box) are not below 2^63: the sum is formed of their halves.
+__device__ __forceinline__ float dr2_words(int4 p, const int hn[3], const int ho[3]) {
+    const int pv[3] = {p.x, p.y, p.z};
+    long long S = 0;
+#pragma unroll
+    for (int a = 0; a < 3; a++) {
+        const long long dn = (int)((uint32_t)pv[a] - (uint32_t)hn[a]), dO = (int)((uint32_t)pv[a] - (uint32_t)ho[a]);
+        S += ((dn - dO) * (dn + dO)) >> 1;
+    }
+    return 2.0f * i64_to_float(S);
+}
+
 // One candidate j against the moved particle: adds u(new) - u(old) to the
 // float accumulator, or to the df accumulator for core pairs.
 template <int MODEL>
@@ -267,14 +282,7 @@ __device__ __forceinline__ void pair_candidate(const Move &m, int4 pj, int tj, c
     const bool near = r2n < near2 || r2o < near2;
     if (MODEL == MODEL_DHLJ && !cn && !co && near) {
         // accurate difference form: u_o expm1(-kappa dr - log1p(dr / r_o))
-        long long S = 0;
-        const int pjv[3] = {pj.x, pj.y, pj.z};
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            long long dn = (int)(pjv[a] - m.hn[a]), dO = (int)(pjv[a] - m.ho[a]);
-            S += (dn - dO) * (dn + dO);
-        }
-        const float dR2 = i64_to_float(S) * d.s32sq;
+        const float dR2 = dr2_words(pj, m.hn, m.ho) * d.s32sq;
         const float ro = sqrtf(r2o), rn = sqrtf(r2n);
         const float dr = dR2 / (rn + ro);
         const float z = fmaf(-d.kappa, dr, -log1pf(dr / ro));
@@ -292,16 +300,9 @@ __device__ __forceinline__ void pair_candidate(const Move &m, int4 pj, int tj, c
         // r_n^2 - r_o^2 = sum_a (dn_a - do_a)(dn_a + do_a) exact in integers
         // (minimum images taken separately, as the reference's sqdist does):
         //   LJ: 4eps x_o^3 (t^3 - 1)(x_o^3 (t^3 + 1) - 1), t = r_o^2 / r_n^2
-        long long S = 0;
-        const int pjv[3] = {pj.x, pj.y, pj.z};
-#pragma unroll
-        for (int a = 0; a < 3; a++) {
-            long long dn = (int)(pjv[a] - m.hn[a]), dO = (int)(pjv[a] - m.ho[a]);
-            S += (dn - dO) * (dn + dO);
-        }
         // DH: u_n/u_o - 1 = (expm1(-kappa dr) - t)/(1 + t), t = dr/r_o, with
         // expm1 by its Taylor series (|kappa dr| is small) or expm1f.
-        const float dR2 = i64_to_float(S) * d.s32sq;
+        const float dR2 = dr2_words(pj, m.hn, m.ho) * d.s32sq;
         const float rio = rsqrt_nr(r2o), rin = rsqrt_nr(r2n);
         const float ro = r2o * rio, rn = r2n * rin;
         const float dr = dR2 * __frcp_rn(rn + ro);

@@ -283,17 +283,12 @@ __device__ __forceinline__ float coul_f(float r, float rc1i, float A5, float B5)
 }
 
 // r_new^2 - r_old^2 (Angstrom^2) from exact integer arithmetic on the high
-// words: sum_a (dn_a - do_a)(dn_a + do_a), each minimum image taken
-// separately as Cuboid::vdist does; |product| < 2^62 always.
+// words, each minimum image taken separately as Cuboid::vdist does.
 __device__ __forceinline__ float dr2_exact(int4 pn, int4 po, int4 pj, const MolDesc &d) {
+    const int hn[3] = {pn.x, pn.y, pn.z}, ho[3] = {po.x, po.y, po.z};
+    if (d.cubic) return fg::dr2_words(pj, hn, ho) * d.s32sq;
     const int dn[3] = {wsub(pn.x, pj.x), wsub(pn.y, pj.y), wsub(pn.z, pj.z)};
     const int dO[3] = {wsub(po.x, pj.x), wsub(po.y, pj.y), wsub(po.z, pj.z)};
-    if (d.cubic) {
-        long long S = 0;
-#pragma unroll
-        for (int a = 0; a < 3; a++) S += ((long long)dn[a] - dO[a]) * ((long long)dn[a] + dO[a]);
-        return fg::i64_to_float(S) * d.s32sq;
-    }
     double S = 0.0;
 #pragma unroll
     for (int a = 0; a < 3; a++)

@@ -73,3 +73,21 @@ def test_systems_in_turns_equal_alone():
         assert per[k]["trials"] == len(streams[k]["u"]) and per[k]["accepted"] == r["acc"].sum()
         for a, b in zip(many[k].state(), alone.state()):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("skew", [False, True])
+def test_molecule_across_the_box(skew):
+    """A molecule moved half the box along every axis: what it leaves and what it
+    meets are a box diagonal's half apart. FP32 terms of the near pairs."""
+    case = dict(m=40, gs=5, box=70.0, dipoles=True, skew=skew)
+    p, x, mu, mus, ids = molecules(case)
+    s, o = MolSystem(p, x, mu, mus, ids, 5), OracleMol(p, x, mu, mus, ids, 5)
+    L = np.array(p.box[:3])
+    rng = np.random.default_rng(6)
+    for g in range(0, 40, 2):
+        new = x.reshape(-1, 5, 3)[g] + L * (0.5 - 0.04 * rng.random(3))
+        new -= L * np.round(new / L)
+        du, ref = s.trial_du(g, new), o.trial_du(g, new)
+        s.commit(False)
+        o.commit(False)
+        assert abs(du - ref) < 4e-6 + 2e-6 * abs(ref), (g, du, ref)

@@ -87,3 +87,26 @@ def test_commit_after_a_batch_run_moved_the_particle(name):
     np.testing.assert_array_equal(r["acc"], ro["acc"])
     # up to 60 near terms of 2 kT, three FP32 roundings each (3e-6), and the reciprocal sum (1e-6)
     assert np.all(np.abs(r["du"] - ro["du"]) < 5e-6 + 1e-9 * np.abs(ro["du"]))
+
+
+@pytest.mark.parametrize("name", list(CASES) + ["octant"])
+def test_far_trials(name):
+    """Particles moved by up to half the box along each axis, a corner's distance
+    among them: the two positions share no partners. Ewald: up to 60 near terms
+    of 2 kT, three FP32 roundings each (3e-6), and the reciprocal sum (1e-6). Salt:
+    the difference form of some four ions within 2 sigma, 1 kT each, off by
+    2e-7 r_o / r_n < 4e-6. Overlaps within 1e-9 of their size."""
+    data = iso() if name == "octant" else CASES[name]()
+    s, o = System(*data), OracleSystem(*data)
+    L, n = data[0].box[0], len(data[1])
+    rng = np.random.default_rng(n + 2)
+    x = s.positions()
+    for t in range(40):
+        i = int(rng.integers(n))
+        step = L * (rng.random(3) - 0.5) if t % 2 else 0.5 * L * (1.0 - 0.05 * rng.random(3))
+        new = x[i] + step
+        new -= L * np.floor(new / L + 0.5)
+        du, ref = s.trial_du(i, new), o.trial_du(i, new)
+        s.commit(False)
+        o.commit(False)
+        assert abs(du - ref) < (1.5e-5 if name.startswith("salt") else 5e-6) + 1e-9 * abs(ref), (t, du, ref)
