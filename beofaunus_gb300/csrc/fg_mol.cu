@@ -73,6 +73,12 @@ constexpr int kMolSiteQueue = 32 * (kMolPerLane + 1);   // a queue of less than 
 constexpr int kMolPairQueue = 256;   // near pairs of a warp (about 110 at C = 16 and 425 at C = 4 for 1000 x 20
                                      // sites; what exceeds it the warp evaluates as it comes)
 constexpr int kMolQueue = 2 * kMolSiteQueue + kMolPairQueue;   // words of a warp: two site queues, near pairs
+// A correction beyond this (kT) belongs to a trial on top of where an accepted
+// molecule was: its dU would be the small rest of two large numbers that a df
+// holds to 2^-46 of their size. It is kept as a NaN, the group ends before a
+// trial that took it, and the next group evaluates the trial (its first) against
+// the configuration as it is.
+constexpr float kMolLargeCorr = 1.0e4f;
 
 // Error bits
 constexpr int kMolErrNonFinite = 8;
@@ -980,6 +986,7 @@ __global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc
                 const int a = e - lo;
                 if (d.trials[cursor + a].g == d.trials[cursor + m].g) continue;
                 df c = uni ? mol_correction<true>(d, s, a, m, s32, L) : mol_correction<false>(d, s, a, m, s32, L);
+                if (!(fabsf(c.hi) <= kMolLargeCorr)) c.hi = __int_as_float(0x7FFFFFFF);
                 c.hi = __shfl_sync(0xffffffffu, c.hi, 0);
                 c.lo = __shfl_sync(0xffffffffu, c.lo, 0);
                 if (CLUSTER) {
@@ -1018,8 +1025,8 @@ __global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc
                     done = a;   // its molecule was moved by an accepted trial of this group
                     break;
                 }
-                if (f & 2) {
-                    bad = 1;
+                if (f & 2) {   // after other trials: perhaps by kMolLargeCorr
+                    bad = a == 0;
                     done = a;
                     break;
                 }

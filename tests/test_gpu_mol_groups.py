@@ -91,3 +91,30 @@ def test_molecule_across_the_box(skew):
         s.commit(False)
         o.commit(False)
         assert abs(du - ref) < 4e-6 + 2e-6 * abs(ref), (g, du, ref)
+
+
+@pytest.mark.parametrize("cluster", [1, 4])
+@pytest.mark.parametrize("off", [0.0, 1e-4, 0.05, 0.3])
+def test_molecule_takes_the_place_of_one_that_left(off, cluster):
+    """A molecule moves onto the sites (or within `off` Angstrom of them) that
+    another left a trial before: nothing of the overlap that the group saw may
+    stay in its dU. A few FP32 roundings of near terms, as above."""
+    gs, m, L = 4, 12, 60.0
+    p, x, mu, mus, ids = workloads.dipolar_molecules(m, seed=3, molsize=gs, box=L)
+    x = x.reshape(m, gs, 3)
+    x[1] = x[0] - x[0, 0] + x[1, 0]   # the same conformation
+    n = 8
+    trans = np.zeros((n, 3))
+    group = np.array([5, 0, 1, 6, 7, 8, 9, 10], np.int32)
+    trans[0] = 0.3, 0.2, 0.1
+    trans[1] = 14.0, 3.0, 2.0
+    trans[2] = x[0, 0] - x[1, 0] + off
+    trans[2] -= L * np.round(trans[2] / L)
+    trans[3:] = 0.1 * np.arange(3, n)[:, None] * np.array([1.0, -1.0, 1.0])
+    st = dict(group=group, axis=np.tile([0.0, 0.0, 1.0], (n, 1)), center=np.zeros(n, np.int32), angle=np.zeros(n),
+              trans=trans, u=np.full(n, 1e-30))
+    x = x.reshape(-1, 3)
+    s = MolSystem(p, x, mu, mus, ids, gs, cluster=cluster)
+    r, ro = s.sweep(st, rotate=False), OracleMol(p, x, mu, mus, ids, gs).run_stream(st, rotate=False)
+    np.testing.assert_array_equal(r["acc"], ro["acc"])
+    assert np.all(np.abs(r["du"] - ro["du"]) < 1e-6 + 4e-7 * np.abs(ro["du"]))
