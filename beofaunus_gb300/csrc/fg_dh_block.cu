@@ -58,12 +58,17 @@ struct BlkSmem {
     float2 *corr;    // [32][32] c(a, m) as df (cluster: two, by block parity)
     float2 *part;    // [32] this CTA's partial sums
     float2 *xpart;   // [2][C][32] every CTA's partial sums (by block parity)
-    int *info;       // [4]: trials resolved in the block, decisions bitmask, queue length
+    int *info;       // [4]: trials resolved in the block, decisions bitmask, queue length, some sum in fix[1], [2]
     uint32_t *queue; // near pairs (trial << 24 | slice index), evaluated densely after the sums
-    unsigned long long *fix;  // [32] near-pair sums per trial, fixed point 2^-40
+    unsigned long long *fix;  // [3][32] near-pair sums per trial (blk_fix_add)
 };
 
-constexpr int kBlkQueue = 1472;
+constexpr int kBlkQueue = 1344;
+// A correction beyond this (kT) belongs to a trial on top of where an accepted
+// particle was: its dU would be the small rest of two large numbers. It is kept
+// as a NaN, the block ends before a trial that took it, and the next block
+// evaluates the trial (its first) as the configuration is.
+constexpr float kBlkLargeCorr = 1.0e4f;
 
 __host__ __device__ inline size_t blk_align(size_t x) { return (x + 15) & ~(size_t)15; }
 
@@ -74,7 +79,7 @@ __host__ __device__ inline size_t blk_smem_bytes(int ns, bool slice, int C) {
     o += blk_align(8 * kBlkTrials) + blk_align(4 * kBlkTrials);
     o += blk_align(8 * kBlkTrials * kBlkTrials) * (C > 1 ? 2 : 1) + blk_align(8 * kBlkTrials) + 16;
     o += blk_align((size_t)8 * 2 * C * kBlkTrials);
-    o += blk_align(4 * kBlkQueue) + blk_align(8 * kBlkTrials);
+    o += blk_align(4 * kBlkQueue) + blk_align(3 * 8 * kBlkTrials);
     return o;
 }
 
@@ -101,17 +106,43 @@ __device__ inline BlkSmem blk_carve(unsigned char *b, int ns, bool slice, int C)
     return s;
 }
 
-// df -> fixed point (2^-40) and back, for order-independent sums of near pairs
-__device__ __forceinline__ unsigned long long blk_to_fix(df v) {
-    const long long a = __float2ll_rn(v.hi * 1099511627776.0f);
-    const long long b = __float2ll_rn(v.lo * 1099511627776.0f);
-    return (unsigned long long)(a + b);
+// Order-independent sums of near pairs in fixed point, by size so that no sum
+// wraps: units of 2^-40 kT below 2^16 kT, 2^-24 below 2^32, 2^-4 for the overlaps
+// beyond, held to 2^53 kT each (128 pairs of the largest size fit 63 bits).
+__device__ __forceinline__ unsigned long long blk_to_fix(df v, float scale) {
+    return (unsigned long long)(__float2ll_rn(v.hi * scale) + __float2ll_rn(v.lo * scale));
 }
-__device__ __forceinline__ df blk_from_fix(unsigned long long u) {
+__device__ __noinline__ void blk_fix_add_large(unsigned long long *fix, df v) {
+    const float x = fabsf(v.hi);
+    if (x < 4294967296.0f) {
+        atomicAdd(fix + kBlkTrials, blk_to_fix(v, 16777216.0f));
+        return;
+    }
+    // (a NaN, of particles on top of each other, counts as the largest overlap)
+    if (!(x < 9007199254740992.0f)) v = df{v.hi < 0.0f ? -9007199254740992.0f : 9007199254740992.0f, 0.0f};
+    atomicAdd(fix + 2 * kBlkTrials, blk_to_fix(v, 16.0f));
+}
+__device__ __forceinline__ void blk_fix_add(const BlkSmem &s, int m, df v) {
+    if (fabsf(v.hi) < 65536.0f) {
+        atomicAdd(&s.fix[m], blk_to_fix(v, 1099511627776.0f));
+    } else {
+        s.info[3] = 1;
+        blk_fix_add_large(&s.fix[m], v);
+    }
+}
+__device__ __forceinline__ df blk_from_fix(unsigned long long u, float scale) {
     const long long v = (long long)u;
     const float h = i64_to_float(v);
     const long long r = v - __float2ll_rn(h);
-    return fast_two_sum(h * 9.094947017729282e-13f, i64_to_float(r) * 9.094947017729282e-13f);
+    return fast_two_sum(h * scale, i64_to_float(r) * scale);
+}
+__device__ __forceinline__ df blk_fix_sum(const BlkSmem &s, int m) {
+    df v = blk_from_fix(s.fix[m], 9.094947017729282e-13f);
+    if (s.info[3]) {
+        v = df_add(v, blk_from_fix(s.fix[kBlkTrials + m], 5.9604644775390625e-8f));
+        v = df_add(v, blk_from_fix(s.fix[2 * kBlkTrials + m], 0.0625f));
+    }
+    return v;
 }
 
 __device__ __forceinline__ float blk_rcp(float x) {
@@ -382,8 +413,8 @@ __global__ void __launch_bounds__(kBlkThreads, 1) dh_block_kernel(const SysDesc 
             if (d.kT != 1.0f) thr = dfm_f(thr, d.kT);
             s.thr[tid] = make_float2(thr.hi, thr.lo);
         }
-        if (tid < kBlkTrials) s.fix[tid] = 0ull;
-        if (tid == 0) s.info[2] = 0;
+        if (tid < 3 * kBlkTrials) s.fix[tid] = 0ull;
+        if (tid == 0) s.info[2] = s.info[3] = 0;
         __syncthreads();
         if (tid < kb) {
             uint32_t c = 0;
@@ -442,13 +473,13 @@ __global__ void __launch_bounds__(kBlkThreads, 1) dh_block_kernel(const SysDesc 
                         ext = SLICE ? s.sext[jj] : d.pos_ext[j];
                     }
                     v = blk_pair(s.mv[m], pj, tj, &ext, d);
-                    if (!live) atomicAdd(&s.fix[m], blk_to_fix(v));
+                    if (!live) blk_fix_add(s, m, v);
                 }
                 const df w = {__shfl_xor_sync(0xffffffffu, v.hi, 1), __shfl_xor_sync(0xffffffffu, v.lo, 1)};
                 if (u < np) {
                     // lane pairs: new minus old; the two lanes share the stores
                     const df c = (u & 1) ? df_add(w, df_neg(v)) : df_add(v, df_neg(w));
-                    const float2 out = make_float2(c.hi, c.lo);
+                    const float2 out = make_float2(fabsf(c.hi) <= kBlkLargeCorr ? c.hi : __int_as_float(0x7FFFFFFF), c.lo);
                     if (CLUSTER) {
                         for (int r = u & 1; r < C; r += 2) blk_st_cluster(&xc[a * kBlkTrials + m], (unsigned)r, out);
                     } else if (!(u & 1)) {
@@ -464,7 +495,7 @@ __global__ void __launch_bounds__(kBlkThreads, 1) dh_block_kernel(const SysDesc 
             const int m = tid & (kBlkTrials - 1), to = tid / kBlkTrials;
             if (m < kb) {
                 const float2 p = s.part[m];
-                const df v = df_add(df{p.x, p.y}, blk_from_fix(s.fix[m]));
+                const df v = df_add(df{p.x, p.y}, blk_fix_sum(s, m));
                 if (CLUSTER) blk_st_cluster(&xp[rank * kBlkTrials + m], (unsigned)to, make_float2(v.hi, v.lo));
                 else xp[m] = make_float2(v.hi, v.lo);
             }
@@ -505,8 +536,14 @@ __global__ void __launch_bounds__(kBlkThreads, 1) dh_block_kernel(const SysDesc 
                 S.hi = add ? Sc.hi : S.hi;
                 S.lo = add ? Sc.lo : S.lo;
             }
+            // kBlkLargeCorr: the sums of the trials before do not depend on the later ones
+            const uint32_t nan = __ballot_sync(0xffffffffu, lane < done && !(S.hi == S.hi));
+            if (nan & ~1u) {
+                done = __ffs(nan & ~1u) - 1;
+                accm &= (1u << done) - 1u;
+            }
             nacc += __popc(accm);
-            if (__any_sync(0xffffffffu, lane < done && !(S.hi == S.hi))) err |= kErrNonFinite;
+            if (nan & 1u) err |= kErrNonFinite;
             // lane m's S is trial m's dU as decided: log it, and add the
             // accepted ones to the running sums (a fixed-order warp sum)
             const bool take = lane < done && ((accm >> lane) & 1u);

@@ -58,3 +58,40 @@ def test_uneven_batch_matches_oracle():
     for s, d, st in zip(batch.systems, data, streams):
         du, acc = s.log_get(0, 200)
         check(du, acc, OracleSystem(*d).mc_run_stream(*st))
+
+
+def overlaps(n):
+    """A stream with trials on top of an ion that stays (0 - 9), of one that left
+    a trial before (20 - 29 follow 10 - 19) and of one of two that overlap from
+    the start (30), among ordinary ones."""
+    p, x, q, ids = salt(n, tables=True)
+    L = p.box[0]
+    rng = np.random.default_rng(n)
+    v = np.array([0.6, -0.5, 0.62])
+    offs = [1.8, 1.2, 0.9, 0.6, 0.4, 0.3, 0.2, 0.1, 0.05, 0.02]
+    x[n - 12] = x[n - 11] + 0.3 * v
+    trials = []   # particle, displacement, uniform
+    for k, r in enumerate(offs):
+        def onto(i, j):
+            d = x[j] + r * v - x[i]
+            return i, d - L * np.round(d / L), 0.5
+        trials += [onto(k, n - 1 - k), (10 + k, np.array([11.0, 9.0, -8.0]), 1e-30), onto(20 + k, 10 + k)]
+        trials += [(32 + 4 * k + m, 2.0 * (rng.random(3) - 0.5), rng.random()) for m in range(4)]
+    trials.append((30, x[n - 11] + 0.25 * v - x[30] - L * np.round((x[n - 11] + 0.25 * v - x[30]) / L), 0.5))
+    trials.append((n - 11, np.array([5.0, 6.0, -7.0]), 0.5))
+    st = np.array([t[0] for t in trials], np.int32), np.array([t[1] for t in trials]), np.array([t[2] for t in trials])
+    return (p, x, q, ids), st
+
+
+@pytest.mark.parametrize("n", [120, 600])   # one CTA and eight
+def test_overlaps(n):
+    """Energies of an overlap are held to 9e15 kT and decide as they should;
+    nothing stays behind of one that is gone. Long steps (1e-6 rms) to
+    six times their rms; coordinates of 48 bits: L / 2^48 of r >= 0.2 Angstrom,
+    times 12, is 1e-11 of the energy."""
+    data, st = overlaps(n)
+    r, ro = System(*data).sweep(*st), OracleSystem(*data).mc_run_stream(*st)
+    np.testing.assert_array_equal(r["acc"], ro["acc"])
+    held = np.abs(ro["du"]) < 9.0e15
+    assert np.all(np.abs(r["du"] - ro["du"])[held] < 6e-6 + 1e-9 * np.abs(ro["du"][held]))
+    assert np.all(r["du"][~held] * np.sign(ro["du"][~held]) > 8.0e15)
