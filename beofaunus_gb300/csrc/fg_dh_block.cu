@@ -40,11 +40,13 @@ struct __align__(16) BlkView {   // one trial
     float wx, wy, wz;      // |d_o| beyond which the image may change
     float qc;              // q lB / (L / 2^32)
     int small;             // kappa |delta| < 1/4: expm1 by its Taylor series
+    int far;               // a step longer than 4 sigma: blk_far_long
     int ti, i;             // type, particle
 };
 struct BlkConst {          // one system
     float kw, kl, near2, s2;   // kappa and -kappa log2(e) per word, 4 sigma^2 and sigma^2 in words^2 (uniform tables)
     float w2;                  // words^2 per Angstrom^2
+    float step2;               // 16 sigma^2 of the smallest pair, words^2
 };
 
 struct BlkSmem {
@@ -162,7 +164,7 @@ __device__ __forceinline__ float blk_ex2(float x) {
 // r_n^2 - r_o^2 = |delta|^2 - 2 delta.d_o for the step delta, and per axis
 // e (2 d_o + e) with e = -delta - 2^32 rint((d_o - delta) / 2^32) where the
 // step may change the minimum image (a warp-uniform branch).
-__device__ __forceinline__ BlkView blk_view(const Move &m, const SysDesc &d) {
+__device__ __forceinline__ BlkView blk_view(const Move &m, const SysDesc &d, float step2) {
     BlkView v;
     v.hx = m.ho[0]; v.hy = m.ho[1]; v.hz = m.ho[2];
     float w[3];
@@ -177,6 +179,7 @@ __device__ __forceinline__ BlkView blk_view(const Move &m, const SysDesc &d) {
     v.ti = m.ti;
     v.i = m.i;
     v.small = d.kappa * d.s32[0] * sqrtf(v.d2) < 0.25f;
+    v.far = !(v.d2 <= step2);
     return v;
 }
 __device__ __forceinline__ float3 blk_diff(const BlkView &v, int4 p) {   // partner - old position, words
@@ -210,7 +213,8 @@ __device__ __forceinline__ float blk_rsqrt(float x) {   // hardware estimate plu
 // (small) difference. UNI: sums d3 and d3 s3 go to l1, l2 (scaled at the end).
 // Straight-line (selects, no branch), so that a warp's two trials interleave.
 // Returns true (adding nothing) for a partner within 2 sigma; `skip` lanes add
-// nothing either.
+// nothing either. For steps of up to 4 sigma only (of the smallest pair): r_n^2
+// as r_o^2 + dR2 loses (r_o / r_n)^2 in relative accuracy, at most 9 there.
 template <bool UNI, bool SMALL>
 __device__ __forceinline__ bool blk_far(const BlkView &v, const BlkConst &c, const SysDesc &d, float3 o, float dR2,
                                         float qj, int tj, bool skip, float &acc, float &l1, float &l2) {
@@ -254,6 +258,31 @@ __device__ __forceinline__ bool blk_far(const BlkView &v, const BlkConst &c, con
     return near && !skip;
 }
 
+// The same for a longer step (qc: the trial's): both distances from their own
+// exact differences and both energies by themselves, since far apart the
+// difference form's error grows with r_o / r_n. rms error of a trial over the
+// whole box, 16384 ions (L = 202 Angstrom): 6.4e-6 kT by blk_far, 3.7e-6 by the
+// difference form on r_n of its own, 3.3e-6 so; steps of up to 40 Angstrom
+// 7.4e-7, 7.4e-7, 6.7e-7. Time per trial as for short steps (0.39 us at 2001
+// ions, 0.85 at 16384).
+__device__ __forceinline__ bool blk_far_long(const Move &m, float qc, const BlkConst &c, int4 p, int tj, const SysDesc &d,
+                                             float &acc) {
+    auto r2_of = [&](const int h[3]) {
+        const float x = (float)(int)((uint32_t)p.x - (uint32_t)h[0]), y = (float)(int)((uint32_t)p.y - (uint32_t)h[1]),
+                    z = (float)(int)((uint32_t)p.z - (uint32_t)h[2]);
+        return fmaf(x, x, fmaf(y, y, z * z));
+    };
+    const float r2n = r2_of(m.hn), r2o = r2_of(m.ho);
+    const int t = d.uniform_types ? 0 : m.ti * d.n_types + tj;
+    const float s2 = d.s2[t] * c.w2;
+    if (fminf(r2n, r2o) < 4.0f * s2) return true;
+    const float rin = blk_rsqrt(r2n), rio = blk_rsqrt(r2o);
+    const float xn = s2 * (rin * rin), xo = s2 * (rio * rio), n3 = xn * xn * xn, o3 = xo * xo * xo;
+    acc = fmaf(qc * __int_as_float(p.w), fmaf(rin, blk_ex2(c.kl * (r2n * rin)), -rio * blk_ex2(c.kl * (r2o * rio))), acc);
+    acc = fmaf(d.eps4[t] * (n3 - o3), n3 + o3 - 1.0f, acc);
+    return false;
+}
+
 // dU contribution of one partner (high words pj with charge bits, type tj,
 // extension e) for trial m, as a df number.
 __device__ __forceinline__ df blk_pair(const Move &m, int4 pj, int tj, const short4 *e, const SysDesc &d) {
@@ -281,6 +310,47 @@ __device__ __forceinline__ bool blk_enqueue(const BlkSmem &s, bool near, uint32_
         return false;
     }
     return true;
+}
+
+// A warp's sums of two trials in one tree: da's in lanes 0..15, db's in 16..31.
+__device__ __forceinline__ df blk_two_sums(df da, df db) {
+    const bool hi = (threadIdx.x & 31) >= 16;   // the half-warps exchange first
+    const df give = hi ? da : db;
+    df sum = hi ? db : da;
+    sum = df_add(sum, df{__shfl_xor_sync(0xffffffffu, give.hi, 16), __shfl_xor_sync(0xffffffffu, give.lo, 16)});
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1)
+        sum = df_add(sum, df{__shfl_xor_sync(0xffffffffu, sum.hi, o), __shfl_xor_sync(0xffffffffu, sum.lo, o)});
+    return sum;
+}
+
+// blk_base for a warp with a step longer than 4 sigma.
+template <bool SLICE>
+__device__ __forceinline__ df blk_base_long(const BlkSmem &s, const SysDesc &d, const BlkConst &c, int ma, int mb, int j0,
+                                            int ns) {
+    const int lane = threadIdx.x & 31;
+    df sum[2] = {{0.0f, 0.0f}, {0.0f, 0.0f}};
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+        const int mm = h ? mb : ma;
+        if (mm < 0) break;
+        const Move &m = s.mv[mm];
+        const int self = m.i - j0;
+        const float qc = s.view[mm].qc;
+        float f = 0.0f;
+        df v = {0.0f, 0.0f};
+        for (int jb = 0; jb < ns; jb += 32) {
+            const int j = jb + lane, k = min(j, ns - 1);
+            const int4 p = SLICE ? s.spos[k] : d.pos4[j0 + k];
+            const int t = SLICE ? s.stype[k] : d.ptype[j0 + k];
+            bool near = false;
+            if (j < ns && j != self) near = blk_far_long(m, qc, c, p, t, d, f);
+            if (__any_sync(0xffffffffu, near) && blk_enqueue(s, near, ((uint32_t)mm << 24) | (uint32_t)j))
+                pair_candidate<MODEL_DHLJ>(m, p, t, SLICE ? &s.sext[k] : &d.pos_ext[j0 + k], d, f, v);
+        }
+        sum[h] = df_add_f(v, f);
+    }
+    return blk_two_sums(sum[0], sum[1]);
 }
 
 // Base sums of the trials ma and mb (mb < 0: none) over the CTA's slice by one
@@ -334,15 +404,7 @@ __device__ __forceinline__ df blk_base(const BlkSmem &s, const SysDesc &d, const
     }
     da = df_add_f(da, fa);
     db = df_add_f(db, fb);
-    // both sums in one tree: the half-warps exchange first
-    const bool hi = lane >= 16;
-    const df give = hi ? da : db;
-    df sum = hi ? db : da;
-    sum = df_add(sum, df{__shfl_xor_sync(0xffffffffu, give.hi, 16), __shfl_xor_sync(0xffffffffu, give.lo, 16)});
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1)
-        sum = df_add(sum, df{__shfl_xor_sync(0xffffffffu, sum.hi, o), __shfl_xor_sync(0xffffffffu, sum.lo, o)});
-    return sum;
+    return blk_two_sums(da, db);
 }
 
 // One cluster of C CTAs per system; system members[blockIdx.x / C] of descs
@@ -385,9 +447,11 @@ __global__ void __launch_bounds__(kBlkThreads, 1) dh_block_kernel(const SysDesc 
     else __syncthreads();
     int64_t nblock = 0;
     const bool uni = d.uniform_types != 0;
+    float s2min = d.s2[0];
+    for (int t = 1; t < d.n_types * d.n_types; t++) s2min = fminf(s2min, d.s2[t]);
     const BlkConst bc = {d.kappa * d.s32[0], -d.kappa * d.s32[0] * 1.4426950408889634f,
                          4.0f * d.s2[0] / (d.s32[0] * d.s32[0]), d.s2[0] / (d.s32[0] * d.s32[0]),
-                         1.0f / (d.s32[0] * d.s32[0])};
+                         1.0f / (d.s32[0] * d.s32[0]), 16.0f * s2min / (d.s32[0] * d.s32[0])};
     // the trial records of the next block are loaded during this one (used if
     // this one resolves all its trials)
     Trial nx{};
@@ -408,7 +472,7 @@ __global__ void __launch_bounds__(kBlkThreads, 1) dh_block_kernel(const SysDesc 
             Move m;
             move_setup(m, tr.idx, xo, xn, __int_as_float(d.pos4[tr.idx].w), d.ptype[tr.idx], d);
             s.mv[tid] = m;
-            s.view[tid] = blk_view(m, d);
+            s.view[tid] = blk_view(m, d, bc.step2);
             df thr = {tr.thr_hi, tr.thr_lo};
             if (d.kT != 1.0f) thr = dfm_f(thr, d.kT);
             s.thr[tid] = make_float2(thr.hi, thr.lo);
@@ -429,7 +493,10 @@ __global__ void __launch_bounds__(kBlkThreads, 1) dh_block_kernel(const SysDesc 
         static_assert(kBlkTrials == 2 * (kBlkThreads / 32), "one turn of two trials per warp");
         if (warp < kb) {
             const int mb = warp + nwarp < kb ? warp + nwarp : -1;
-            const df p = uni ? blk_base<SLICE, true>(s, d, bc, warp, mb, j0, ns) : blk_base<SLICE, false>(s, d, bc, warp, mb, j0, ns);
+            const bool far = s.view[warp].far || s.view[mb < 0 ? warp : mb].far;
+            const df p = far   ? blk_base_long<SLICE>(s, d, bc, warp, mb, j0, ns)
+                         : uni ? blk_base<SLICE, true>(s, d, bc, warp, mb, j0, ns)
+                               : blk_base<SLICE, false>(s, d, bc, warp, mb, j0, ns);
             if (lane == 0) s.part[warp] = make_float2(p.hi, p.lo);
             if (lane == 16 && mb >= 0) s.part[mb] = make_float2(p.hi, p.lo);
         }

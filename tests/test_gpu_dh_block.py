@@ -95,3 +95,21 @@ def test_overlaps(n):
     held = np.abs(ro["du"]) < 9.0e15
     assert np.all(np.abs(r["du"] - ro["du"])[held] < 6e-6 + 1e-9 * np.abs(ro["du"][held]))
     assert np.all(r["du"][~held] * np.sign(ro["du"][~held]) > 8.0e15)
+
+
+@pytest.mark.parametrize("n,dp,rms", [(500, 40.0, 1.0e-6), (2001, 40.0, 1.0e-6), (500, 1e9, 1.6e-6), (2001, 1e9, 2.5e-6), (16384, 1e9, 5.0e-6)])
+def test_long_steps(n, dp, rms):
+    """Steps of up to 40 Angstrom and of any length. Some four near pairs (within
+    2 sigma) of 0.75 kT, in difference form, are off by 1.2e-7 r_o / r_n each: with
+    r_o / r_n = 18 over the box of 16384 ions 3.4e-6 together, in proportion less
+    in smaller boxes; far pairs, each energy by itself, add 3e-7 (6e-6 where r_n
+    came from r_o). Trials on top of another ion are left to test_overlaps."""
+    p, x, q, ids = salt(n)
+    dp = min(dp, p.box[0])
+    st = stream(n, 900, 3 * n, dp)
+    keep = OracleSystem(p, x, q, ids).mc_run_stream(*st)["du"] < 10.0   # rejected trials leave the chain as it is
+    st = tuple(np.ascontiguousarray(a[keep]) for a in st)
+    s, o = System(p, x, q, ids), OracleSystem(p, x, q, ids)
+    r, ro = s.sweep(*st), o.mc_run_stream(*st)
+    np.testing.assert_array_equal(r["acc"], ro["acc"])
+    assert np.sqrt(np.mean((r["du"] - ro["du"]) ** 2)) < rms
