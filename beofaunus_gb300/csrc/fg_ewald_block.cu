@@ -31,6 +31,11 @@ constexpr int kEbTrials = 32;
 constexpr int kEbThreads = 512;
 constexpr int kEbKc = 128;   // scratch buffer rows (of 32 float2)
 constexpr int kEbMaxCluster = 16;
+// A correction beyond this (kT) belongs to a trial on top of where an accepted
+// particle was: its dU would be the small rest of two large numbers. It is kept
+// as a NaN, the block ends before a trial that took it, and the next block
+// evaluates the trial (its first) as the configuration is.
+constexpr float kEbLargeCorr = 1.0e4f;
 constexpr int kEbGramN = 6 * 32 * 4;   // floats of one Gram accumulator set (eb_gram_regs' layout)
 
 struct EbSmem {
@@ -1044,7 +1049,8 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
                 }
                 const df w = {__shfl_xor_sync(0xffffffffu, v.hi, 1), __shfl_xor_sync(0xffffffffu, v.lo, 1)};
                 if (u < np && !(u & 1)) {
-                    const df c = df_add(v, df_neg(w));
+                    df c = df_add(v, df_neg(w));
+                    if (!(fabsf(c.hi) <= kEbLargeCorr)) c.hi = __int_as_float(0x7FFFFFFF);
                     float2 *to = &s.corr[a * kEbTrials + m];
                     if (CLUSTER) eb_st_remote(to, 0, make_float2(c.hi, c.lo));
                     else *to = make_float2(c.hi, c.lo);
@@ -1277,8 +1283,9 @@ __global__ void __launch_bounds__(kEbThreads, 1) ewald_block_kernel(const SysDes
                 S.hi = add ? Sc.hi : S.hi;
                 S.lo = add ? Sc.lo : S.lo;
             }
-            // a trial whose particle an accepted one moved ends the block
-            const uint32_t again = __ballot_sync(0xffffffffu, (colm & accm) != 0u);
+            // a trial whose particle an accepted one moved ends the block, and so does kEbLargeCorr
+            const bool nan = lane > 0 && lane < kb && !(S.hi == S.hi);
+            const uint32_t again = __ballot_sync(0xffffffffu, (colm & accm) != 0u || nan);
             if (again) done = __ffs(again) - 1;
             if (done < 32) accm &= (1u << done) - 1u;
             if (__popc(accm) >= left) {   // and so does the accepted one that makes a rebuild due

@@ -60,3 +60,28 @@ def test_block_sweep_matches_oracle(name, ctas):
     assert np.all((np.abs(r["du"] - ro["du"]) < bound)[judged])
     d = s.positions() - o.positions()
     assert np.abs(d - box * np.round(d / box)).max() < 1e-9
+
+
+@pytest.mark.parametrize("ctas", [1, 4])
+@pytest.mark.parametrize("kappa", [False, True])
+def test_place_of_an_ion_that_left(ctas, kappa):
+    """Ions that move onto the place that another left a trial before: nothing
+    of the overlap that the block saw may stay in their dU."""
+    n, box = 200, 40.0
+    p, x, q, ids = workloads.rpm_ewald(n, box, 5, 8, cutoff=19.0, start="scatter")
+    if kappa:
+        p.ewald_debye_length = 15.0
+    rng = np.random.default_rng(9)
+    trials = []
+    for k, r in enumerate([1.0, 0.5, 0.2, 0.1, 0.03, 0.01, 1e-3, 1e-5, 0.0]):
+        onto = x[10 + k] + r - x[30 + k]
+        trials += [(10 + k, np.array([11.0, 9.0, -8.0]), 1e-30), (30 + k, onto - box * np.round(onto / box), 0.5)]
+        trials += [(50 + 4 * k + m, 2.0 * (rng.random(3) - 0.5), rng.random()) for m in range(4)]
+    st = np.array([t[0] for t in trials], np.int32), np.array([t[1] for t in trials]), np.array([t[2] for t in trials])
+    s, o = System(p, x, q, ids), OracleSystem(p, x, q, ids)
+    s.cluster = ctas
+    r, ro = s.sweep(*st), o.mc_run_stream(*st)
+    np.testing.assert_array_equal(r["acc"], ro["acc"])
+    bound = (TOL_KAPPA if kappa else TOL) + 1e-9 * np.abs(ro["du"])
+    judged = np.abs(ro["du"]) < 10.0 if kappa else slice(None)   # as above
+    assert np.all((np.abs(r["du"] - ro["du"]) < bound)[judged])
