@@ -54,6 +54,8 @@
 // image of every pair; the others (19 % at 1000 molecules in 150 A) are
 // collected and take min(|dx|, L - |dx|) for LJ and the exact integer
 // difference for ion-dipole, which is odd in r.
+#include "fg_mol_turns.h"
+
 namespace fgm {
 
 using fg::df;
@@ -1626,33 +1628,10 @@ int mol_run(fg_molsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
     else L.fn = L.cluster ? fgm::mol_sweep_kernel<false, true, false> : fgm::mol_sweep_kernel<false, false, false>;
     CK(cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
     if (L.cluster) CK(cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    // A last wave of clusters that is nearly empty costs as much as a full one
-    // (at C = 4 the GPU holds 36 clusters at once: 38 systems ran 2 waves for
-    // 1.06 waves' work). Where more than a tenth would be lost, the systems
-    // take turns: launches of exactly `slots` clusters run `quantum` trials of
-    // each, in rotation, so that all of them are full.
     const int64_t kChunk = 65536;   // most trials of one launch
-    int slots = n;
-    int64_t quantum = kChunk;
-    const int fit = mol_slots(h0, L);
-    if (fit > 0 && fit < n) {
-        const int waves = (n + fit - 1) / fit;
-        if (10 * n < 9 * waves * fit) {
-            double best = waves;
-            for (int q = 2; q <= 16; q++) {   // turns per system; whole groups each
-                const int64_t qu = ((maxn + q - 1) / q + fgm::kMolAhead - 1) / fgm::kMolAhead * fgm::kMolAhead;
-                const int64_t turns = (maxn + qu - 1) / qu, rounds = (turns * n + fit - 1) / fit;
-                // in waves of maxn trials; a launch lasts as long as its unluckiest system, whose
-                // groups ended early on a molecule met twice (about 6 trials at 1000 molecules)
-                const double cost = (double)rounds * (qu + 6) / maxn;
-                if (qu <= kChunk && cost < best) {
-                    best = cost;
-                    slots = fit;
-                    quantum = qu;
-                }
-            }
-        }
-    }
+    const fgm::MolTurns turns = fgm::mol_turns(maxn, n, mol_slots(h0, L), fgm::kMolAhead, kChunk);
+    const int slots = turns.slots;
+    const int64_t quantum = turns.quantum;
     cudaStream_t st = h0->stream;
     const fgm::MolDesc *descs = h0->d_desc;
     if (h0->run_cap < n) {

@@ -118,3 +118,12 @@ def test_molecule_takes_the_place_of_one_that_left(off, cluster):
     r, ro = s.sweep(st, rotate=False), OracleMol(p, x, mu, mus, ids, gs).run_stream(st, rotate=False)
     np.testing.assert_array_equal(r["acc"], ro["acc"])
     assert np.all(np.abs(r["du"] - ro["du"]) < 1e-6 + 4e-7 * np.abs(ro["du"]))
+
+
+def test_empty_streams_of_more_systems_than_fit():
+    p, x, mu, mus, ids = workloads.dipolar_molecules(20, seed=1, molsize=6)
+    many = [MolSystem(p, x, mu, mus, ids, 6, cluster=4) for _ in range(41)]
+    for s in many[::2]:   # staged with no trial, or never staged
+        s.stream_upload(mol_draw_stream(1, 20, 0))
+    per, tot = mol_run_many(many)
+    assert tot["trials"] == 0 and all(q["trials"] == 0 and q["accepted"] == 0 for q in per)
