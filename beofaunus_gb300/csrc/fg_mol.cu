@@ -205,7 +205,7 @@ struct GroupBuf {
 
 struct MolSmem {
     int4 *spos;     // site slice: high words, .w = type
-    float4 *sdip;   // dipole slice: mu-hat * mu, mu
+    float4 *sdip;   // dipole slice: mu-hat * mu, mu (in global memory where it does not fit)
     int4 *sdpos;    // dipole slice positions, .w = site << 8 | type
     unsigned char *groups;   // `ahead` group buffers
     uint32_t *queue;   // [kMolWarps][kMolQueue]: a warp's sites that may change image, near sites, near pairs
@@ -916,7 +916,7 @@ __device__ __noinline__ df mol_correction(const MolDesc &d, const MolSmem &sm, i
 // over several warps.
 template <bool SLICE_SMEM, bool CLUSTER, bool EVAL>
 __global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc *__restrict__ descs, int ahead,
-                                                                  int64_t quantum) {
+                                                                  int dips, int64_t quantum) {
     extern __shared__ __align__(16) unsigned char mol_smem_raw[];
     const int C = CLUSTER ? (int)descs[0].C : 1;
     const int sys = blockIdx.x / C;
@@ -931,10 +931,15 @@ __global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc
     const int ns_full = (d.N + C - 1) / C, nd_full = (d.D + C - 1) / C;
     const int j0 = min(rank * ns_full, d.N), j1 = min(j0 + ns_full, d.N), ns = j1 - j0;
     const int k0 = min(rank * nd_full, d.D), k1 = min(k0 + nd_full, d.D), nd = k1 - k0;
-    MolSmem s = mol_carve(mol_smem_raw, ns_full, nd_full, d.gs, SLICE_SMEM, ahead);
+    const bool dip_smem = SLICE_SMEM || dips;
+    MolSmem s = mol_carve(mol_smem_raw, ns_full, dip_smem ? nd_full : 0, d.gs, SLICE_SMEM, ahead);
+    if (!dip_smem) {
+        s.sdip = d.dip4 + k0;
+        s.sdpos = d.dip_pos4 + k0;
+    }
     if (SLICE_SMEM)
         for (int jj = tid; jj < ns; jj += blockDim.x) s.spos[jj] = d.pos4[j0 + jj];
-    for (int kk = tid; kk < nd; kk += blockDim.x) {
+    for (int kk = tid; dip_smem && kk < nd; kk += blockDim.x) {
         s.sdip[kk] = d.dip4[k0 + kk];
         s.sdpos[kk] = d.dip_pos4[k0 + kk];
     }
@@ -1099,7 +1104,7 @@ __global__ void __launch_bounds__(kMolThreads, 1) mol_sweep_kernel(const MolDesc
     if (!EVAL) {
         if (SLICE_SMEM)
             for (int jj = tid; jj < ns; jj += blockDim.x) d.pos4[j0 + jj] = s.spos[jj];
-        for (int kk = tid; kk < nd; kk += blockDim.x) {
+        for (int kk = tid; dip_smem && kk < nd; kk += blockDim.x) {
             d.dip4[k0 + kk] = s.sdip[kk];
             d.dip_pos4[k0 + kk] = s.sdpos[kk];
         }
@@ -1340,40 +1345,43 @@ void mol_mass_center(const int64_t *X, int front, int gs, int64_t out[3]) {
 }
 
 constexpr size_t kMolSmemMax = 220 * 1024;   // of the 227 KB a CTA may hold
-size_t mol_smem_bytes(const fg_molsys *h, int C, bool slice_smem, int ahead) {
+// What a launch keeps in shared memory beside the queues.
+struct MolFit {
+    bool slice;   // the site slice
+    bool dips;    // the dipole slice
+    int ahead;    // trials per group
+};
+size_t mol_smem_bytes(const fg_molsys *h, int C, const MolFit &f) {
     size_t off[16];
-    fgm::mol_smem_layout((h->N + C - 1) / C, (h->D + C - 1) / C, h->gs, slice_smem, ahead, off);
+    fgm::mol_smem_layout((h->N + C - 1) / C, f.dips ? (h->D + C - 1) / C : 0, h->gs, f.slice, f.ahead, off);
     return off[7];
 }
-// Trials per group of a launch: kMolAhead where their buffers fit beside the
-// site slice, fewer (at least four) where that keeps the slice in shared
-// memory; slice = false: the slice stays in global memory (one buffer where
-// the dipole slice leaves room for no more).
-int mol_ahead(const fg_molsys *h, int C, bool &slice) {
-    slice = true;
+// Trials per group: kMolAhead where their buffers fit beside the slices, fewer
+// (at least four) where that keeps the site slice in shared memory; else it
+// stays in global memory, and so does the dipole slice where it leaves no room
+// for one trial (from some 5500 sites with a dipole in a CTA on).
+MolFit mol_fit(const fg_molsys *h, int C) {
     for (int a = fgm::kMolAhead; a >= 4; a /= 2)
-        if (mol_smem_bytes(h, C, true, a) <= kMolSmemMax) return a;
-    slice = false;
-    int a = fgm::kMolAhead;
-    while (a > 1 && mol_smem_bytes(h, C, false, a) > kMolSmemMax) a /= 2;
-    return a;
+        if (mol_smem_bytes(h, C, {true, true, a}) <= kMolSmemMax) return {true, true, a};
+    for (int a = fgm::kMolAhead; a >= 1; a /= 2)
+        if (mol_smem_bytes(h, C, {false, true, a}) <= kMolSmemMax) return {false, true, a};
+    return {false, false, fgm::kMolAhead};
 }
 
 struct MolLaunch {
-    void (*fn)(const fgm::MolDesc *, int, int64_t);
+    void (*fn)(const fgm::MolDesc *, int, int, int64_t);
     size_t smem;
-    int ahead;
+    MolFit fit;
     bool cluster;
 };
 
 template <bool EVAL>
 int mol_pick(const fg_molsys *h, MolLaunch &L) {
-    bool slice;
-    L.ahead = mol_ahead(h, h->C, slice);
+    L.fit = mol_fit(h, h->C);
     const bool cl = h->C > 1;
-    L.smem = mol_smem_bytes(h, h->C, slice, L.ahead);
+    L.smem = mol_smem_bytes(h, h->C, L.fit);
     L.cluster = cl;
-    if (slice) L.fn = cl ? fgm::mol_sweep_kernel<true, true, EVAL> : fgm::mol_sweep_kernel<true, false, EVAL>;
+    if (L.fit.slice) L.fn = cl ? fgm::mol_sweep_kernel<true, true, EVAL> : fgm::mol_sweep_kernel<true, false, EVAL>;
     else L.fn = cl ? fgm::mol_sweep_kernel<false, true, EVAL> : fgm::mol_sweep_kernel<false, false, EVAL>;
     cudaError_t e = cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem);
     if (e != cudaSuccess) return fail(FG_ERR_CUDA, "shared memory attribute: %s", cudaGetErrorString(e));
@@ -1400,7 +1408,7 @@ int mol_launch(const fg_molsys *h, const MolLaunch &L, const fgm::MolDesc *descs
         cfg.attrs = attr;
         cfg.numAttrs = 1;
     }
-    cudaError_t e = cudaLaunchKernelEx(&cfg, L.fn, descs, L.ahead, quantum);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, L.fn, descs, L.fit.ahead, L.fit.dips ? 1 : 0, quantum);
     if (e != cudaSuccess) return fail(FG_ERR_CUDA, "molecule sweep launch: %s", cudaGetErrorString(e));
     return FG_OK;
 }
@@ -1604,27 +1612,24 @@ int mol_upload(fg_molsys *h, int64_t n, const int32_t *mol, const double *axis, 
 int mol_run(fg_molsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *total) {
     if (!sys || n < 1) return fail(FG_ERR_INVALID, "bad argument");
     fg_molsys *h0 = sys[0];
-    bool all_slice = true;
-    int ahead = fgm::kMolAhead;   // group buffers that fit every system
+    MolFit fit{true, true, fgm::kMolAhead};   // what fits for every system
     int64_t maxn = 0;
     for (int i = 0; i < n; i++) {
         fg_molsys *h = sys[i];
         if (!h || !h->state_set) return fail(FG_ERR_STATE, "system %d has no state", i);
         if (h->C != h0->C) return fail(FG_ERR_INVALID, "systems must share the cluster size");
         if (h->device != h0->device) return fail(FG_ERR_INVALID, "systems must share the device");
-        bool slice;
-        const int a = mol_ahead(h, h->C, slice);
-        if (!slice) all_slice = false;
-        ahead = std::min(ahead, a);
+        const MolFit f = mol_fit(h, h->C);
+        fit = {fit.slice && f.slice, fit.dips && f.dips, std::min(fit.ahead, f.ahead)};
         maxn = std::max(maxn, h->n_stream);
         CK(cudaStreamSynchronize(h->stream));
     }
     MolLaunch L;
     L.cluster = h0->C > 1;
-    L.ahead = ahead;
+    L.fit = fit;
     L.smem = 0;
-    for (int i = 0; i < n; i++) L.smem = std::max(L.smem, mol_smem_bytes(sys[i], sys[i]->C, all_slice, ahead));
-    if (all_slice) L.fn = L.cluster ? fgm::mol_sweep_kernel<true, true, false> : fgm::mol_sweep_kernel<true, false, false>;
+    for (int i = 0; i < n; i++) L.smem = std::max(L.smem, mol_smem_bytes(sys[i], sys[i]->C, fit));
+    if (fit.slice) L.fn = L.cluster ? fgm::mol_sweep_kernel<true, true, false> : fgm::mol_sweep_kernel<true, false, false>;
     else L.fn = L.cluster ? fgm::mol_sweep_kernel<false, true, false> : fgm::mol_sweep_kernel<false, false, false>;
     CK(cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
     if (L.cluster) CK(cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));

@@ -127,3 +127,22 @@ def test_empty_streams_of_more_systems_than_fit():
         s.stream_upload(mol_draw_stream(1, 20, 0))
     per, tot = mol_run_many(many)
     assert tot["trials"] == 0 and all(q["trials"] == 0 and q["accepted"] == 0 for q in per)
+
+
+@pytest.mark.parametrize("m", [176, 192, 208])   # 5456, 5952 and 6448 sites with a dipole on one CTA
+def test_dipole_slices_up_to_the_shared_memory(m):
+    p, x, mu, mus, ids = molecules(dict(m=m // 8, gs=31, box=57.5, dipoles=True))
+    cells = np.array([[a, b, c] for a in (0, 1) for b in (0, 1) for c in (0, 1)]) * 57.5 - 28.75
+    x, mu, mus, ids = (x[None] + cells[:, None]).reshape(-1, 3), np.tile(mu, (8, 1)), np.full(31 * m, 0.3), np.tile(ids, 8)
+    for a in range(3):
+        p.box[a] = 115.0
+    s, o = MolSystem(p, x, mu, mus, ids, 31, cluster=1), OracleMol(p, x, mu, mus, ids, 31)
+    st = mol_draw_stream(5, m, 40, 1.0, 0.3, True)
+    r, ro = s.sweep(st), o.run_stream(st)
+    np.testing.assert_array_equal(r["acc"], ro["acc"])
+    # 31 x 31 dipole pairs with a close molecule instead of a few: four times the bound of the grouped sweeps;
+    # overlaps (up to 1e10 kT): six times r^2's rounding (1.5e-7) in r^-12, twice
+    assert np.all(np.abs(r["du"] - ro["du"]) < 4e-6 + 2e-6 * np.abs(ro["du"]))
+    new = s.state()[0].reshape(m, 31, 3)[3] + 0.4
+    assert abs(s.trial_du(3, new) - o.trial_du(3, new)) < 4e-6
+    s.commit(False)
