@@ -259,8 +259,18 @@ __global__ void energy64_qk_sum_kernel(const double2 *__restrict__ part, int nch
 
 namespace {
 
-// The FP64 energy's and the g(r) sampling's device workspace: kept with the
-// system (freed with it), grown when a call needs more.
+// The FP64 energy's and the g(r) sampling's device workspace: grown when a call
+// needs more, and kept with the system (freed with it) up to kWork64Keep: a
+// batch may ask every member for its energy.
+constexpr size_t kWork64Keep = (size_t)4 << 20;
+constexpr size_t kWork64Qk = (size_t)3 << 20;   // Q(k) partial sums for which more chunks are taken
+void drop_work64(fg_system *h) {   // after the call's last synchronisation
+    if (h->work64_cap <= kWork64Keep) return;
+    cudaFree(h->work64);
+    h->work64 = nullptr;
+    h->device_bytes -= h->work64_cap;
+    h->work64_cap = 0;
+}
 int ensure_work64(fg_system *h, size_t bytes) {
     if (bytes <= h->work64_cap) return FG_OK;
     if (h->work64) {
@@ -308,11 +318,14 @@ int total_energy_fp64_boxes(fg_system *h, int nbox, const double (*boxes)[3], do
         }
     std::vector<double> qe(N);
     for (int j = 0; j < N; j++) qe[j] = h->charges[j] * eff[h->types[j]];
-    // pair tiles over at most kE64MaxBlocks blocks; Q(k) chunks of particles
-    // so that a few blocks per SM share the work
+    // pair tiles over at most kE64MaxBlocks blocks; Q(k) chunks of at most 1024
+    // particles, whole stages, and as many as their partial sums fit kWork64Qk
+    // (8192 ions, K = 1152: 128 chunks of two stages)
     const long long nti = (N + fg::kE64Threads - 1) / fg::kE64Threads, ntj = (N + fg::kE64Tile - 1) / fg::kE64Tile;
     const int nb = (int)std::min<long long>(fg::kE64MaxBlocks, nti * ntj);
-    const int chunk = std::max(fg::kE64Stage, (N + 511) / 512), nchunk = K > 0 ? (N + chunk - 1) / chunk : 0;
+    const int most = std::max((N + 1023) / 1024, K > 0 ? (int)std::min<size_t>(512, kWork64Qk / ((size_t)K * sizeof(double2))) : 1);
+    const int chunk = ((N + most - 1) / most + fg::kE64Stage - 1) / fg::kE64Stage * fg::kE64Stage;
+    const int nchunk = K > 0 ? (N + chunk - 1) / chunk : 0;
     // one workspace, kept with the system and grown when needed: q, qe, pair
     // tables, partial sums, |Q(k)|^2, Q(k) partial sums
     auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -364,6 +377,7 @@ int total_energy_fp64_boxes(fg_system *h, int nbox, const double (*boxes)[3], do
     CK(cudaMemcpyAsync(part.data(), d_part, part.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     if (K > 0) CK(cudaMemcpyAsync(q2.data(), d_q2, K * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    drop_work64(h);
     double M0[3] = {0, 0, 0};  // sum q eff x in the current box
     if (K > 0) {
         std::vector<double> xyz(3 * (size_t)N);

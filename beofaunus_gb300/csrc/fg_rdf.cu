@@ -115,6 +115,7 @@ extern "C" int fg_rdf_sample(fg_system *h, int32_t type1, int32_t type2, double 
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(out.data(), d_buf, bytes, cudaMemcpyDeviceToHost, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    drop_work64(h);
     for (int b = 0; b < n_bins; b++) hist[b] += (int64_t)out[b];
     if (n_pairs) *n_pairs += (int64_t)out[n_bins];
     return FG_OK;

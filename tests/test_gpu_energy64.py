@@ -39,3 +39,16 @@ def test_fp64_energy_and_rdf_at_tile_edges(model, n, box):
         ho, to = atom_rdf_counts(pos, ids, list(p.box), t1, t2, dr, bins)
         assert t == to
         np.testing.assert_array_equal(h, ho)
+
+
+def test_energy_workspace_is_bounded():
+    """What a system keeps for its FP64 energy and g(r): at most 4 MB, also with
+    512 chunks' worth of particles and 2242 k-vectors."""
+    from beofaunus_gb300.gpu import System
+    p, x, q, ids = workloads.rpm_ewald(16384, 164.0, 10, 1, start="scatter")
+    s = System(p, x, q, ids)
+    before = s.device_bytes
+    e = s.total_energy_fp64()
+    s.rdf_sample(0, 1, 0.25, 90)
+    assert s.device_bytes - before <= 4 << 20
+    assert s.total_energy_fp64() == e
