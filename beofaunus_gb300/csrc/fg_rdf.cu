@@ -15,10 +15,10 @@
 // take the FP64 form, so every count is the FP64 one. 8192 ions: 6.0 ms -> 75 us
 // per call (FP64 for every pair on 32 blocks before); bound by the pair loop's
 // issue rate and the shared-memory atomics.
+#include "fg_rdf_grid.h"
+
 namespace fg {
 
-constexpr int kRdfThreads = 128;
-constexpr int kRdfTile = 128;        // j positions staged per pass
 constexpr int kRdfMaxBins = 8192;    // shared-memory histogram (uint32)
 
 __global__ void __launch_bounds__(kRdfThreads) rdf_kernel(const SysDesc *__restrict__ dsc, int t1, int t2,
@@ -104,8 +104,7 @@ extern "C" int fg_rdf_sample(fg_system *h, int32_t type1, int32_t type2, double 
     CK(cudaMemsetAsync(d_buf, 0, bytes, h->stream));
     double unit = 0;
     for (int a = 0; a < 3; a++) unit = std::max(unit, std::ldexp(h->P.box[a], -32));
-    const long long nt = (h->N + fg::kRdfThreads - 1) / fg::kRdfThreads;
-    const int blocks = (int)std::min<long long>(nt * nt, 8LL * dh_sm_count());
+    const int blocks = (int)fg::rdf_blocks(h->N, dh_sm_count());
     fg::rdf_kernel<<<blocks, fg::kRdfThreads, (size_t)n_bins * sizeof(uint32_t), h->stream>>>(
         h->d_desc, type1, type2,
         make_double3(std::ldexp(h->P.box[0], -64), std::ldexp(h->P.box[1], -64), std::ldexp(h->P.box[2], -64)),
