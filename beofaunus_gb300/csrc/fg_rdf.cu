@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(kRdfThreads) rdf_kernel(const SysDesc *__restr
     for (int b = tid; b < n_bins; b += blockDim.x) h[b] = 0u;
     if (tid == 0) cnt = 0ull;
     const int nti = (N + kRdfThreads - 1) / kRdfThreads, ntj = (N + kRdfTile - 1) / kRdfTile;
-    const float idr = (float)inv_dr;
+    const float idr = (float)fmin(inv_dr, 1e30);   // (finite: with smaller dr every pair takes the FP64 form)
     unsigned mine = 0;
     for (long long t = blockIdx.x; t < (long long)nti * ntj; t += gridDim.x) {
         const int i0 = (int)(t / ntj) * kRdfThreads, j0 = (int)(t % ntj) * kRdfTile;

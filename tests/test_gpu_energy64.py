@@ -52,3 +52,16 @@ def test_energy_workspace_is_bounded():
     s.rdf_sample(0, 1, 0.25, 90)
     assert s.device_bytes - before <= 4 << 20
     assert s.total_energy_fp64() == e
+
+
+@pytest.mark.parametrize("dr", [1e-20, 1e-35, 1e-39, 1e-45, 1e-300])
+def test_rdf_bins_far_below_single_precision(dr):
+    """Two ions in one place count in bin 0 at any bin width, the others nowhere."""
+    from beofaunus_gb300.gpu import System
+    p, x, q, ids = system("salt", 257)
+    x[2] = x[0]   # both of type 0
+    ids[0] = ids[2] = 0
+    s = System(p, x, q, ids)
+    h, t = s.rdf_sample(0, 0, dr, 4)
+    n = int((ids == 0).sum())
+    assert t == n * (n - 1) // 2 and list(h) == [1, 0, 0, 0]
