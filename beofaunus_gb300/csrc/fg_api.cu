@@ -1575,8 +1575,9 @@ int fg_trial_du(fg_system *h, int32_t n_moved, const int32_t *idx, const double 
     cfg.numAttrs = cfg.gridDim.x > 1 ? 1 : 0;
     CK(cudaLaunchKernelEx(&cfg, trial_fn(h), (const SysDesc *)h->d_desc, a, h->trial_out,
                           (volatile unsigned long long *)h->trial_host));
-    // dU arrives in pinned memory; a synchronisation (and its error, if any)
-    // only if it has not within a few milliseconds
+    // dU arrives in pinned memory, after some 20 us; a call that waits longer
+    // (behind other work on the GPU) synchronises, as the device's scheduling
+    // flags say, and so gets its error, if any
     unsigned long long w[2];
     bool synced = false;
     const auto t0 = std::chrono::steady_clock::now();
@@ -1584,7 +1585,7 @@ int fg_trial_du(fg_system *h, int32_t n_moved, const int32_t *idx, const double 
         for (int x = 0; x < 2; x++) w[x] = __atomic_load_n(&h->trial_host[x], __ATOMIC_ACQUIRE);
         if ((uint32_t)(w[0] >> 32) == a.call && (uint32_t)(w[1] >> 32) == a.call) break;
         if (synced) return fail(FG_ERR_DEVICE, "the trial's result did not arrive");
-        if ((spin & 1023) == 1023 && std::chrono::steady_clock::now() - t0 > std::chrono::milliseconds(5)) {
+        if ((spin & 255) == 255 && std::chrono::steady_clock::now() - t0 > std::chrono::microseconds(200)) {
             CK(cudaStreamSynchronize(h->stream));
             synced = true;
         }
