@@ -1048,9 +1048,10 @@ int dip_dmalloc(fg_dipsys *h, void **p, size_t bytes) {
 
 int dip_push_desc(fg_dipsys *h) {
     if (h->has_pushed && !std::memcmp(&h->pushed, &h->desc, sizeof(fgd::DipDesc))) return FG_OK;
+    h->has_pushed = false;   // until the copy has gone out
+    CK(cudaMemcpyAsync(h->d_desc, &h->desc, sizeof(fgd::DipDesc), cudaMemcpyHostToDevice, h->stream));
     std::memcpy(&h->pushed, &h->desc, sizeof(fgd::DipDesc));
     h->has_pushed = true;
-    CK(cudaMemcpyAsync(h->d_desc, &h->desc, sizeof(fgd::DipDesc), cudaMemcpyHostToDevice, h->stream));
     return FG_OK;
 }
 

@@ -1482,10 +1482,11 @@ int mol_alloc_replicas(fg_molsys *h, int C) {
 int mol_push_desc(fg_molsys *h) {
     h->desc.C = h->C;
     if (h->has_pushed && !std::memcmp(&h->pushed, &h->desc, sizeof(fgm::MolDesc))) return FG_OK;
-    std::memcpy(&h->pushed, &h->desc, sizeof(fgm::MolDesc));
-    h->has_pushed = true;
+    h->has_pushed = false;   // until the copy has gone out
     CK(cudaMemcpyAsync(h->d_desc, &h->desc, sizeof(fgm::MolDesc), cudaMemcpyHostToDevice, h->stream));
     CK(cudaStreamSynchronize(h->stream));
+    std::memcpy(&h->pushed, &h->desc, sizeof(fgm::MolDesc));
+    h->has_pushed = true;
     return FG_OK;
 }
 
