@@ -1615,6 +1615,7 @@ int mol_run(fg_molsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
     fg_molsys *h0 = sys[0];
     MolFit fit{true, true, fgm::kMolAhead};   // what fits for every system
     int64_t maxn = 0;
+    int fewest = INT32_MAX;   // molecules of the smallest system
     for (int i = 0; i < n; i++) {
         fg_molsys *h = sys[i];
         if (!h || !h->state_set) return fail(FG_ERR_STATE, "system %d has no state", i);
@@ -1623,6 +1624,7 @@ int mol_run(fg_molsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
         const MolFit f = mol_fit(h, h->C);
         fit = {fit.slice && f.slice, fit.dips && f.dips, std::min(fit.ahead, f.ahead)};
         maxn = std::max(maxn, h->n_stream);
+        fewest = std::min(fewest, h->M);
         CK(cudaStreamSynchronize(h->stream));
     }
     MolLaunch L;
@@ -1635,7 +1637,7 @@ int mol_run(fg_molsys *const *sys, int n, fg_sweep_stats *per, fg_sweep_stats *t
     CK(cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem));
     if (L.cluster) CK(cudaFuncSetAttribute((const void *)L.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     const int64_t kChunk = 65536;   // most trials of one launch
-    const fgm::MolTurns turns = fgm::mol_turns(maxn, n, mol_slots(h0, L), fgm::kMolAhead, kChunk);
+    const fgm::MolTurns turns = fgm::mol_turns(maxn, n, mol_slots(h0, L), fgm::kMolAhead, fewest, kChunk);
     const int slots = turns.slots;
     const int64_t quantum = turns.quantum;
     cudaStream_t st = h0->stream;

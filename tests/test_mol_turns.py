@@ -12,7 +12,7 @@ MAIN = r"""
 #include <cstdlib>
 #include "fg_mol_turns.h"
 int main(int, char **v) {
-    const fgm::MolTurns t = fgm::mol_turns(std::atoll(v[1]), std::atoi(v[2]), std::atoi(v[3]), 16, 65536);
+    const fgm::MolTurns t = fgm::mol_turns(std::atoll(v[1]), std::atoi(v[2]), std::atoi(v[3]), 16, std::atoi(v[4]), 65536);
     std::printf("%d %lld\n", t.slots, (long long)t.quantum);
 }
 """
@@ -25,8 +25,8 @@ def turns(tmp_path_factory):
     subprocess.run(["g++", "-std=c++17", "-O1", "-fsanitize=undefined", "-fno-sanitize-recover=all",
                     "-I" + os.path.join(ROOT, "beofaunus_gb300", "csrc"), "-o", str(d / "main"), str(d / "main.cpp")], check=True)
 
-    def run(*args):
-        r = subprocess.run([str(d / "main")] + [str(a) for a in args], capture_output=True, text=True)
+    def run(maxn, n, fit, molecules=1000):
+        r = subprocess.run([str(d / "main"), str(maxn), str(n), str(fit), str(molecules)], capture_output=True, text=True)
         assert r.returncode == 0, r.stderr
         return tuple(int(x) for x in r.stdout.split())
     return run
@@ -49,3 +49,11 @@ def test_every_system_gets_all_its_turns(turns, n, maxn):
         per = -(-maxn // quantum)
         rounds = -(-per * n // slots)
         assert rounds * slots >= per * n
+
+
+@pytest.mark.parametrize("molecules,trials,take", [(1000, 64, False), (1000, 256, True), (200, 64, False), (200, 256, True),
+                                                   (200, 1024, True), (60, 64, False), (60, 1024, True), (24, 256, True),
+                                                   (2, 16, False)])
+def test_turns_where_they_were_faster(turns, molecules, trials, take):
+    """38 systems on 36 slots, as measured (mol_turns); never for one group."""
+    assert (turns(trials, 38, 36, molecules)[0] == 36) == take
