@@ -543,12 +543,6 @@ __global__ void __launch_bounds__(kDipMaxThreads, 1) dip_build_kernel(const DipD
     dip_rebuild(d, A, S, before, after);
 }
 
-// mode 0: run the staged stream [cursor, n_trials) with Metropolis decisions;
-// mode 1: evaluate trials[0] (explicit) and keep it pending;
-// mode 2: apply the pending trials[0] as accepted.
-// MAXT: the launch bound. 128 threads per system at most 128 registers
-// (four systems, sixteen warps on an SM) or up to kDipMaxThreads at one CTA
-// per SM.
 // A newly staged stream: cursor, per-stream sum and flags from zero.
 __global__ void dip_begin_kernel(DipScalars *sc) {
     sc->cursor = 0;
@@ -577,6 +571,12 @@ __global__ void dip_gather_kernel(const DipDesc *descs, int n, DipScalars *out) 
     if (i < n) out[i] = *descs[i].sc;
 }
 
+// mode 0: run the staged stream [cursor, n_trials) with Metropolis decisions;
+// mode 1: evaluate trials[0] (explicit) and keep it pending;
+// mode 2: apply the pending trials[0] as accepted.
+// MAXT: the launch bound. 128 threads per system at most 128 registers
+// (four systems, sixteen warps on an SM) or up to kDipMaxThreads at one CTA
+// per SM.
 template <int MAXT>
 __global__ void __launch_bounds__(MAXT, MAXT <= 128 ? 4 : 1) dip_sweep_kernel(const DipDesc *__restrict__ descs, int mode,
                                                                                int stage) {

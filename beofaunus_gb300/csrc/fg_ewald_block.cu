@@ -12,11 +12,11 @@
 //   reciprocal   sum_k A'_k 2 Re(conj(D_a,k) D_m,k)
 // with D_m,k = q (e^{ik.r_new} - e^{ik.r_old}) = 2 q sin(k.d / 2) i e^{ik.r_mid},
 // r_mid the step's midpoint, the same increment the energy uses (its error is
-// relative to |d|, and a real sine times a phase takes 10 of the 65 slots that
-// q e^{ik.r_old}(e^{ik.d} - 1) took less).
+// relative to |d|; a real sine times a phase takes 55 issue slots, the form
+// q e^{ik.r_old}(e^{ik.d} - 1) took 65).
 // The reciprocal parts of all pairs of the block form a 32 x 32 Gram matrix
-// over k of the trials' increments; it is accumulated in 4 x 4 register tiles
-// while the increments stream through shared memory in chunks of k-vectors.
+// over k of the trials' increments; the warps accumulate it on the tensor cores
+// (eb_gram_regs), each from the increments that it forms in registers.
 // Q(k) itself stays the exact fixed-point sum: after the block each accepted
 // trial's integer contributions are applied in order. A trial whose particle
 // an accepted trial of the block already moved ends the block, and so does
@@ -119,8 +119,6 @@ __device__ inline EbSmem eb_carve(char *base, const SysDesc &d, bool cells) {
     return s;
 }
 
-// Real-space sum of one trial by one warp: every stencil cell (cell list) or
-// every particle (no cell list), lanes over the slots.
 // One k-step of the Gram matrix on the tensor cores: components c = the real
 // and imaginary parts of 4 consecutive k-vectors of X = sqrt(A') D. mma.sync
 // m16n8k8 TF32 with the three-product split (hi hi + hi lo + lo hi, each

@@ -110,7 +110,6 @@ struct MolScalars {
 struct alignas(16) MolDesc {
     int32_t N, gs, M, D, nt, C, uniform_lj, cubic;
     float s32[3];       // L / 2^32 (one unit of the high word)
-    float sc9[3];       // 512 L / 2^32 (unit of the high word >> 9)
     double s64d[3];     // L / 2^64
     double inv64d[3];   // 2^64 / L
     float lB, rc2, rc2near, rc1i, A5, B5, kT, rfB;
@@ -165,9 +164,6 @@ __device__ __forceinline__ void st_cluster_f2(float2 *p, unsigned rank, float2 v
 // ---------------------------------------------------------------- helpers
 // a - b with two's-complement wrap (the minimum image of high words).
 __device__ __forceinline__ int wsub(int a, int b) { return (int)((uint32_t)a - (uint32_t)b); }
-
-// Exact float of |m| < 2^22 without the conversion pipe.
-__device__ __forceinline__ float small_to_float(int m) { return __int_as_float(0x4B400000 + m) - 12582912.0f; }
 
 struct D3 {
     double x, y, z;
@@ -1757,7 +1753,6 @@ int fg_mol_create(const fg_params *params, int32_t n_sites, int32_t sites_per_mo
     d.uniform_lj = uniform ? 1 : 0;
     for (int a = 0; a < 3; a++) {
         d.s32[a] = (float)(P.box[a] / 4294967296.0);
-        d.sc9[a] = (float)(512.0 * P.box[a] / 4294967296.0);
         d.s32sqd[a] = (P.box[a] / 4294967296.0) * (P.box[a] / 4294967296.0);
         d.s64d[a] = P.box[a] / TWO64;
         d.inv64d[a] = TWO64 / P.box[a];
