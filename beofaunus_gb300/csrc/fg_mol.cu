@@ -1918,6 +1918,7 @@ int fg_mol_set_state(fg_molsys *h, const double *xyz, const double *mu_unit, con
     const float2 u = split_df(tot[0] + tot[1]);
     s.utot_hi = u.x;
     s.utot_lo = u.y;
+    s.n_trials = h->n_stream;   // the stream that is staged runs on the new state, from its first trial
     rc = mol_write_scalars(h, s);
     if (rc) return rc;
     h->pending = -1;

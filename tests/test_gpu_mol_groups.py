@@ -146,3 +146,16 @@ def test_dipole_slices_up_to_the_shared_memory(m):
     new = s.state()[0].reshape(m, 31, 3)[3] + 0.4
     assert abs(s.trial_du(3, new) - o.trial_du(3, new)) < 4e-6
     s.commit(False)
+
+
+def test_a_staged_stream_runs_on_the_state_set_after_it():
+    p, x, mu, mus, ids = molecules(CASES[0])
+    st = mol_draw_stream(3, 3, 60, 1.0, 0.3, True)
+    s = MolSystem(p, x, mu, mus, ids, 20, cluster=1)
+    s.stream_upload(st)
+    y = x + 1.25                       # the same molecules, shifted
+    s.set_state(y, mu, mus, ids)
+    per, _ = mol_run_many([s])
+    ro = OracleMol(p, y, mu, mus, ids, 20).run_stream(st)
+    assert per[0]["trials"] == 60 and per[0]["accepted"] == ro["acc"].sum()
+    assert abs(per[0]["energy_change"] - ro["usum"]) < 60e-6
