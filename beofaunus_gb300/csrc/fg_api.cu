@@ -577,7 +577,7 @@ int size_class(int N) {
 // as keep at least 64 particles each. A block of 32 trials costs about 0.33 us
 // per trial on any number of CTAs and 0.4 ns per particle of a CTA's slice, so
 // more CTAs always help down to slices of 64 (us per trial, 1 / 4 / 16 CTAs:
-// 256 particles 0.67 / 0.49 / -, 2001 1.29 / 0.54 / 0.38, 16384 8.9 / 2.0 / 0.72).
+// 256 particles 0.66 / 0.49 / -, 2001 1.29 / 0.54 / 0.37, 16384 9.1 / 2.0 / 0.71).
 constexpr int kDhMinPerCta = 64;
 int dh_block_ctas(int N) {
     const int maxc = dh_block_max_cluster();

@@ -28,7 +28,7 @@
 // 28 cycles of the SFU per 32 partners), a fixed part of about 0.3 us per
 // trial (near pairs, corrections, barrier, resolution) on small ones. Base sums
 // of 2001 particles on one CTA: 210 -> 120 cycles per warp of partners and SM
-// quarter; per trial 2.24 -> 1.29 us on one CTA, 0.62 -> 0.36 us on 16.
+// quarter; per trial 2.24 -> 1.29 us on one CTA, 0.62 -> 0.38 us on 16.
 namespace fg {
 
 constexpr int kBlkTrials = 32;
