@@ -1231,7 +1231,7 @@ int fg_create(const fg_params *params, int32_t n_particles, fg_system **out) {
     ALLOC(h->sc, sizeof(SysScalars));
     ALLOC(h->ticket, sizeof(unsigned));
     if (cudaMemsetAsync(h->ticket, 0, sizeof(unsigned), h->stream) != cudaSuccess) return bail(fail(FG_ERR_CUDA, "ticket"));
-    ALLOC(h->trial_out, 4 * sizeof(float2));
+    ALLOC(h->trial_out, sizeof(float2));
     ALLOC(h->corr, 4 * sizeof(float2));
     ALLOC(h->sc_tab, 256 * sizeof(float2));
     ALLOC(h->dp_fix, FG_MAX_TYPES * 3 * sizeof(int64_t));

@@ -1018,10 +1018,7 @@ __global__ void __launch_bounds__(kTrialThreads) trial_kernel(const SysDesc *__r
         const unsigned long long call = (unsigned long long)a.call << 32;
         host[0] = call | __float_as_uint(du.hi);
         host[1] = call | __float_as_uint(du.lo);
-        // for the commit
-        out[0] = make_float2(du.hi, du.lo);
-        out[1] = make_float2(dM[0], dM[1]);
-        out[2] = make_float2(dM[2], 0.0f);
+        *out = make_float2(du.hi, du.lo);   // for the commit
     }
 }
 
@@ -1068,8 +1065,9 @@ __device__ __forceinline__ void commit_position_global(const Move &m, const SysD
 
 // Movebase acceptMove + NonbondedEwald::update for the last plain trial. The
 // particle's old position is the one it has now: a batch run between the trial
-// and its commit may have moved it, and Q(k) and the cell lists must lose the
-// position that they hold. The k-vectors spread over the grid, and every CTA
+// and its commit may have moved it, and Q(k), the surface dipole and the cell
+// lists must lose the position that they hold (the energy counts the dU that the
+// trial reported). The k-vectors spread over the grid, and every CTA
 // reads that position; so the last warp of the CTA that is last to have read it
 // (ticket, left at zero) commits the new one and the sums, while the others
 // update Q(k). 4.7 -> 3.1 us at 783 k-vectors, against staging k-vectors and
@@ -1111,7 +1109,7 @@ __global__ void __launch_bounds__(kTrialThreads) commit_kernel(const SysDesc *__
     if (last) {
         commit_position_global(m, d, CELLS);
         SysScalars *sc = d.sc;
-        const df du = {trial_out[0].x, trial_out[0].y};
+        const df du = {trial_out->x, trial_out->y};
         df U = df_add(df{sc->u_hi, sc->u_lo}, du);
         df Ut = df_add(df{sc->utot_hi, sc->utot_lo}, du);
         sc->u_hi = U.hi;
@@ -1120,7 +1118,9 @@ __global__ void __launch_bounds__(kTrialThreads) commit_kernel(const SysDesc *__
         sc->utot_lo = Ut.lo;
         sc->n_accepted++;
         if (KSPACE) {
-            const float dM[3] = {trial_out[1].x, trial_out[1].y, trial_out[2].x};
+            const df M0[3] = {};
+            float dM[3];
+            surface_delta(m, d, M0, dM);
             for (int x = 0; x < 3; x++) {
                 const df ma = df_add_f(df{sc->m[x][0], sc->m[x][1]}, dM[x]);
                 sc->m[x][0] = ma.hi;

@@ -54,11 +54,14 @@ def test_trials_and_commits(name):
         assert s.rebuild_qk() == 0.0   # exact: the rebuild finds what the commits kept
 
 
-@pytest.mark.parametrize("name", ["rpm 240", "rpm 3000 cells", "salt 1030"])
-def test_commit_after_a_batch_run_moved_the_particle(name):
+@pytest.mark.parametrize("name,vacuum", [("rpm 240", False), ("rpm 240", True), ("rpm 3000 cells", False), ("salt 1030", False)])
+def test_commit_after_a_batch_run_moved_the_particle(name, vacuum):
     """The commit takes the particle from where it is, not from where it was
-    when the trial was evaluated: positions, exact Q(k) and cell lists hold."""
+    when the trial was evaluated: positions, exact Q(k), cell lists and the
+    surface dipole (its energy counts in vacuum) hold."""
     data = CASES[name]()
+    if vacuum:
+        data[0].ewald_eps_surf = 1.0
     s, o = System(*data), OracleSystem(*data)
     L, n = data[0].box[0], len(data[1])
     rng = np.random.default_rng(n + 1)
